@@ -333,7 +333,12 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       sidx[q] = col;
       note(k, q, col);
     }
-    if (!__all_sync(0xffffffffu, i == len)) {
+    // rows of the slice longer than kWideSlice; where they are few, a row's
+    // sum stops at its own length (wide_row), which needs its entries in the
+    // first slots
+    const int nlong = __popc(__ballot_sync(0xffffffffu, len > kWideSlice));
+    const bool few_long = w > kWideSlice && nlong <= kWideRows;
+    if (!__all_sync(0xffffffffu, i == len) || few_long) {
       all = true;
       my_d = 0;
       for (int k = 0; k < w; ++k) {
@@ -356,14 +361,12 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       kd8[(long long)s * kNarrow + lane] = d;
       kd8h[(long long)s * kNarrow + lane] = (int16_t)d;  // read only when every |d| < 32768
     }
-    // rows of the slice longer than kWideSlice
-    const int nlong = __popc(__ballot_sync(0xffffffffu, len > kWideSlice));
     if (lane == 0) {
       int f = all ? 1 : 0;
       if (narrow) f |= 2 | (w << 3);
       // a full slice made wide by a few long rows: listed for the solver's
       // pre-pass (wide[0] counts, wide[1 + i] = slice)
-      if (allow_wide && w > kWideSlice && nlong <= kWideRows && 32 * s + 32 <= n) {
+      if (allow_wide && few_long && 32 * s + 32 <= n) {
         const int wi = atomicAdd(wide, 1);
         wide[1 + wi] = s;
         f |= 4 | (wi << 3);
