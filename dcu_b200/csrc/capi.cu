@@ -325,7 +325,9 @@ int autotune(Ctx* c, int n, int nnz, const int* ptr, const int* idx, const doubl
                       (eff ? v.grid_p == 0 && v.grid_y == 0 : v.grid_py == 0);
     if (!same) cands.push_back(v);
   };
-  if (c->profile_k1_free) {
+  if (c->profile_one_launch) {
+    // (the solve runs as one launch, which none of these settings changes)
+  } else if (c->profile_k1_free) {
     add(1);
     add(0);
   } else {
@@ -346,6 +348,7 @@ int autotune(Ctx* c, int n, int nnz, const int* ptr, const int* idx, const doubl
   }
   const int iters = si.iters > 0 ? si.iters : 1;
   t->k1_split = cands[pick].k1_split;
+  if (c->profile_one_launch && c->profile_k1_free) t->k1_split = c->profile_default_split;
   t->grid_p = cands[pick].grid_p;
   t->grid_y = cands[pick].grid_y;
   t->grid_py = cands[pick].grid_py;

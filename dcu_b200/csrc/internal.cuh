@@ -61,6 +61,7 @@ enum BufId {
   B_SELL_MVAL8,    // M values (FP32 / BF16) of the narrow slices, 8 per row, row-major
   B_SELL_AVAL32,   // A values in SELL order, FP32 copy (used when every value is exact in FP32)
   B_SELL_AFLAG,    // int: nonzero when some A value is not exactly an FP32 number
+  B_PERSIST,       // one-launch solver: result, barrier slots, gathered vectors
   B_COUNT
 };
 
@@ -117,6 +118,7 @@ struct Ctx {
   std::vector<int> profile_sel;    // and the grid selector each ran with
   bool profile_k1_free = false;    // fused and split first steps compute the same values
   int profile_default_split = 0;   // the form's default first step
+  bool profile_one_launch = false; // the last solve ran as one launch (persist.cu)
   int plan_wide = 0;               // slices of the last SELL plan wider than kWideSlice
   bool wide_prepass = true;        // flag wide slices for the pre-pass (dcu_set_wide_prepass)
   bool exact_a32 = true;           // A read from its FP32 copy when exact (dcu_set_exact_a32)
@@ -204,6 +206,26 @@ struct SellPlan {
   const int* rptr = nullptr;  // CSR row pointers of the laid-out operator (row lengths)
   const int* wide = nullptr;  // the slices flagged wide (device)
   int nwide = 0;
+  // one-launch solver (persist.cu): most slots and most long rows any of its
+  // blocks holds; 0 slots when it does not take an operator of this size
+  int max_block_slots = 0, max_block_long = 0;
+};
+
+// How the one-launch solver splits an operator of n rows: `blocks` blocks
+// (0: too large for it) of `spb` 32-row slices each.
+struct PersistShape {
+  bool cluster = false;
+  int spb = 0, blocks = 0;
+};
+constexpr int kPersistLong = 16;     // a longer row of a wide slice is summed by a warp
+constexpr int kPersistBlocks = 160;  // most blocks (a multiple of 32)
+PersistShape persist_shape(const Ctx* c, int n);
+
+// What the one-launch solver writes at its end.
+struct SolveOut {
+  double res, true_res, bnorm;
+  int it, status, replacements, a32;
+  int err;
 };
 
 // Slot counts of the last SELL plan built on a context (diagnostics).
@@ -300,6 +322,12 @@ int bicgstab_solve(Ctx* c, const SellPlan& plan, const SellA& aval_sell, const v
                    const double* b, double* x, const dcu_options* opt, dcu_solve_info* info,
                    const void* mval8_sell = nullptr);
 void release_graphs(Ctx* c);
+// The whole solve in one launch, for operators that stay on the chip; *ran
+// tells whether the operator was taken (x, *out and the end event c->ev[1]
+// are then final).  mkind: M's type in mval / mval8, 0 FP64, 1 FP32, 2 BF16.
+// Forms with FP64 vectors only.
+int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* mval, const void* mval8, int mkind,
+                  const double* b, double* x, const dcu_options* opt, bool* ran, SolveOut* out);
 
 // Batched systems (diagonal blocks [sys_off[s], sys_off[s+1]) of one matrix).
 int check_blocks(Ctx* c, int n, const int* ptr, const int* idx, int nsys, const int* sys_off);

@@ -284,7 +284,7 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
                               int* __restrict__ sidx, int* __restrict__ sperm, int* __restrict__ maxdelta,
                               int16_t* __restrict__ del, int* __restrict__ kd, int* __restrict__ su,
                               unsigned long long* __restrict__ uslots, int* __restrict__ wide, int allow_wide,
-                              int* __restrict__ kd8, int16_t* __restrict__ kd8h) {
+                              int* __restrict__ kd8, int16_t* __restrict__ kd8h, int* __restrict__ cost, int spb) {
   __shared__ unsigned long long blk_uslots;
   if (threadIdx.x == 0) blk_uslots = 0ull;
   __syncthreads();
@@ -334,8 +334,8 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       note(k, q, col);
     }
     // rows of the slice longer than kWideSlice; where they are few, a row's
-    // sum stops at its own length (wide_row), which needs its entries in the
-    // first slots
+    // sum stops at its own length (wide_row, the one-launch solver's long
+    // rows), which needs its entries in the first slots
     const int nlong = __popc(__ballot_sync(0xffffffffu, len > kWideSlice));
     const bool few_long = w > kWideSlice && nlong <= kWideRows;
     if (!__all_sync(0xffffffffu, i == len) || few_long) {
@@ -360,6 +360,18 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       const int d = (narrow && lane < w) ? my_d : 0;
       kd8[(long long)s * kNarrow + lane] = d;
       kd8h[(long long)s * kNarrow + lane] = (int16_t)d;  // read only when every |d| < 32768
+    }
+    // the slice's share of a block of the one-launch solver (persist.cu, which
+    // makes the same split): slots kept, entries and number of the long rows
+    if (spb > 0) {
+      const bool split = w > kPersistLong && few_long;
+      const int ws = __reduce_max_sync(0xffffffffu, !split ? w : (len <= kPersistLong ? len : 0));
+      const int le = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? len : 0);
+      const int nl = __popc(__ballot_sync(0xffffffffu, split && len > kPersistLong));
+      if (lane == 0) {
+        atomicAdd(&cost[2 * (s / spb)], 32 * ws + le);
+        if (nl) atomicAdd(&cost[2 * (s / spb) + 1], nl);
+      }
     }
     if (lane == 0) {
       int f = all ? 1 : 0;
@@ -683,10 +695,14 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_TRY(ensure(c, B_SELL_KD, sizeof(int) * ((size_t)nslices + (size_t)(slots / 32) + 1)));
   int* su = bp<int>(c, B_SELL_KD);
   int* kd = su + nslices;
-  DCU_TRY(ensure(c, B_PLANSTAT, 2 * sizeof(unsigned long long)));
+  // slots, uniform slots; then per block of the one-launch solver its slots and long rows
+  const PersistShape ps = persist_shape(c, n);
+  unsigned long long hst[2 + kPersistBlocks] = {(unsigned long long)slots};
+  const size_t nst = sizeof(unsigned long long) * (2 + (size_t)ps.blocks);
+  DCU_TRY(ensure(c, B_PLANSTAT, sizeof(hst)));
   unsigned long long* pst = bp<unsigned long long>(c, B_PLANSTAT);
-  const unsigned long long hst[2] = {(unsigned long long)slots, 0ull};
-  DCU_CUDA(c, cudaMemcpyAsync(pst, hst, sizeof(hst), cudaMemcpyHostToDevice, c->stream));
+  int* cost = reinterpret_cast<int*>(pst + 2);
+  DCU_CUDA(c, cudaMemcpyAsync(pst, hst, nst, cudaMemcpyHostToDevice, c->stream));
   DCU_TRY(ensure(c, B_SELL_WIDE, sizeof(int) * ((size_t)nslices + 1)));
   int* wide = bp<int>(c, B_SELL_WIDE);
   DCU_TRY(ensure(c, B_SELL_KD8, (sizeof(int) + sizeof(int16_t)) * kNarrow * (size_t)nslices));
@@ -695,8 +711,12 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_CUDA(c, cudaMemsetAsync(wide, 0, sizeof(int), c->stream));
   k_sell_layout<<<waves_grid(c, (long long)nslices * 32, 256, 8), 256, 0, c->stream>>>(
       rptr, rcol, rperm, n, nslices, off, sidx, sperm, maxdelta, del, kd, su, pst + 1, wide, c->wide_prepass ? 1 : 0,
-      kd8, kd8h);
+      kd8, kd8h, cost, ps.blocks > 0 ? ps.spb : 0);
   DCU_LAUNCHED(c, "k_sell_layout");
+  int* hcost = reinterpret_cast<int*>(c->pinned) + 4;
+  static_assert(sizeof(int) * (4 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
+  if (ps.blocks > 0)
+    DCU_CUDA(c, cudaMemcpyAsync(hcost, cost, sizeof(int) * 2 * (size_t)ps.blocks, cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(c->pinned, wide, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(reinterpret_cast<int*>(c->pinned) + 1, maxdelta, sizeof(int), cudaMemcpyDeviceToHost,
                               c->stream));
@@ -706,6 +726,11 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_CUDA(c, cudaStreamSynchronize(c->stream));
   if (check_out) *check_out = check ? reinterpret_cast<int*>(c->pinned)[2] : 0;
   plan->nwide = *reinterpret_cast<int*>(c->pinned);
+  plan->max_block_slots = plan->max_block_long = 0;
+  for (int g = 0; g < ps.blocks; ++g) {
+    plan->max_block_slots = std::max(plan->max_block_slots, hcost[2 * g]);
+    plan->max_block_long = std::max(plan->max_block_long, hcost[2 * g + 1]);
+  }
   plan->delta16 = reinterpret_cast<int*>(c->pinned)[1] < 32768;
   plan->del = plan->delta16 ? del : nullptr;
   if (!plan->delta16) kd8h = nullptr;

@@ -292,6 +292,8 @@ int dcu_batch_solve_d(dcu_spai_ctx* ctx, int nsys, const int* sys_off, int n, in
  *   p/y = M p | A y + (r*, Ay) | s/z = M s | A z + dots | x/r update + dots
  * with a narrow (FP32 / BF16) preconditioner six, the first one split in two:
  *   p = r + beta (p - omega Ay) | y = M p | ... (as above)
+ * (a solve that ran as one launch is profiled by the same kernels on its
+ * buffers).
  * *count (optional) receives the number of kernels; DCU_ERR_ARG when cap is
  * smaller.  The solver vectors and x are left in an unspecified state. */
 int dcu_profile_iteration_kernels(dcu_spai_ctx* ctx, int reps, float* ms_out, int cap, int* count);
@@ -350,6 +352,9 @@ int dcu_set_exact_a32(dcu_spai_ctx* ctx, int enabled);
  *              0 = what fits the CTA's shared memory; -1 = no limit (every
  *              block on one CTA, larger ones from a per-CTA global slab).
  *              Changes M by rounding only.
+ * Operators that stay on the chip (up to a few hundred thousand rows; forms
+ * with FP64 vectors) solve in one launch, which the iteration fields do not
+ * change.
  * The report fields are written by dcu_autotune_d and ignored on input. */
 typedef struct {
   int k1_split;
