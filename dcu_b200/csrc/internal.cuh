@@ -61,6 +61,7 @@ enum BufId {
   B_SELL_MVAL8,    // M values (FP32 / BF16) of the narrow slices, 8 per row, row-major
   B_SELL_AVAL32,   // A values in SELL order, FP32 copy (used when every value is exact in FP32)
   B_SELL_AFLAG,    // int: nonzero when some A value is not exactly an FP32 number
+  B_MIDLIST,       // columns for the second and third size of the FP64 group kernel
   B_PERSIST,       // one-launch solver: result, barrier slots, gathered vectors
   B_COUNT
 };

@@ -56,6 +56,8 @@ enum {
   ST_STAGE_FAIL = 13, // a bulk copy into shared memory did not complete in time
   ST_STAGED = 16,     // CTA-kernel columns whose J columns were staged by bulk copies
   ST_HUB_COUNT = 17,  // columns handed to the hub kernels
+  ST_MID_COUNT = 22,  // columns handed to the second size of the FP64 group kernel
+  ST_WIDE_COUNT = 23, // and to its third
   ST_INTS = 24,
   ST_AREA64 = 7,      // long long index (ints 14-15): max candidates * (|J|+1) over queued columns
   ST_AREASUM64 = 9,   // long long index (ints 18-19): sum of (candidates + 2) * (|J|+1) over queued columns
@@ -451,6 +453,422 @@ __global__ void __launch_bounds__(SG_BLOCK, 12) k_spai_small(SmallArgs a) {
   }
 }
 
+
+// ---------------------------------------------------------------------------
+// FP64 builds: G lanes per column, rows of [At | e_E] spread over the lanes.
+//
+// Householder QR in FP64 is bound by the FP64 pipe and by the chain of each
+// step (norm, square root, reciprocal, dot products, update), so the columns in
+// flight and the work they share per instruction decide.  Here a lane holds
+// RP rows of every column of [At | e_E] (row = lane + G i): each step's dot
+// products with all trailing columns are summed by all G lanes at once (log2 G
+// shuffles a value), nothing is idle but the padding rows, and a warp's 32 / G
+// columns run in lockstep through one unrolled step loop.  (Two lanes per
+// column of [At | e_E], the layout of k_spai_small, leaves the lanes of finished
+// columns idle and re-reads v from shared memory: 4.6 ms at 128^3 on one B200,
+// this one 1.1 ms.)  I_k: the candidate rows of A(:, J) are sorted across the
+// group (bitonic network in registers) and ranked; At is scattered into shared
+// memory and read back by rows.
+//
+// Three sizes (rows, |J|, candidates): every stencil and mesh column stays on a
+// group; the CTA kernel keeps what is larger (a CTA per column, one at a time
+// on an SM: 57% of the columns of a 9-point mesh used to go there, 3.1 ms
+// for 90000 columns).
+//   GroupA  4 lanes, |J| <= 7,  |I| <= 28, <= 64 candidates (2D / 3D stencils)
+//   GroupB  8 lanes, |J| <= 11, |I| <= 32, <= 128           (9-point meshes)
+//   GroupC 16 lanes, |J| <= 15, |I| <= 64, <= 256
+// A column that does not fit is queued for the next size, the last for the CTA
+// kernel.
+// ---------------------------------------------------------------------------
+template <int G_, int NJ_, int RMAX_, int PER_>
+struct GroupShape {
+  static constexpr int G = G_, NJ = NJ_, RMAX = RMAX_, PER = PER_;
+  static constexpr int NC = NJ + 1;           // columns of [At | e_E], e_E last
+  static constexpr int CMAX = G * PER;        // candidates: PER per lane
+  static constexpr int GPW = 32 / G;          // columns per warp
+  static constexpr int LD = NC | 1;           // row stride of At (odd: rows in different banks)
+};
+using GroupA = GroupShape<4, 7, 28, 16>;
+using GroupB = GroupShape<8, 11, 32, 16>;
+using GroupC = GroupShape<16, 15, 64, 16>;
+constexpr int GR_BLOCK = 64;
+
+struct GroupArgs {
+  SmallArgs a;
+  int* mid_list;   // GroupB's columns, or null: what GroupA cannot take goes to the CTA kernel
+  int* wide_list;  // GroupC's columns
+  const int* in;   // this kernel's columns (null: the range) ...
+  int in_count;    // ... and the stats[] entry that counts them
+};
+
+template <typename T, typename S>
+struct GroupSmemRaw {
+  T At[S::RMAX * S::LD];
+  unsigned rows[S::RMAX];   // I_k
+  int base[S::NJ + 1];      // start of J column j in A's arrays, minus its first candidate
+  int cb[S::NJ + 1];        // first candidate of J column j
+  int E;
+};
+// padded so that the groups of a warp start 8 banks apart
+template <typename T, typename S>
+struct alignas(8) GroupSmem : GroupSmemRaw<T, S> {
+  static constexpr int words = (int)(sizeof(GroupSmemRaw<T, S>) / 4);
+  static constexpr int more = (40 - words % 32) % 32;
+  int pad[more ? more : 32];
+};
+
+template <int G, int PER>
+__device__ __forceinline__ void rows_sort(unsigned (&key)[PER], int lane) {
+  constexpr int N = G * PER;
+#pragma unroll
+  for (int kk = 2; kk <= N; kk <<= 1) {
+#pragma unroll
+    for (int jj = kk >> 1; jj > 0; jj >>= 1) {
+      if (jj >= PER) {
+        // ascending block and lower half, or neither: keep the smaller
+        const bool small = (((lane * PER) & kk) == 0) == (((lane * PER) & jj) == 0);
+#pragma unroll
+        for (int s = 0; s < PER; ++s) {
+          const unsigned other = __shfl_xor_sync(0xffffffffu, key[s], jj / PER, G);
+          key[s] = small ? min(key[s], other) : max(key[s], other);
+        }
+      } else {
+#pragma unroll
+        for (int s = 0; s < PER; ++s) {
+          const int p = s ^ jj;
+          if (p > s) {
+            const unsigned x = key[s], y = key[p];
+            const bool up = (kk < PER) ? (s & kk) == 0 : ((lane * PER) & kk) == 0;
+            key[s] = up ? min(x, y) : max(x, y);
+            key[p] = up ? max(x, y) : min(x, y);
+          }
+        }
+      }
+    }
+  }
+}
+
+// An addition that is never contracted with a product before it: a column's
+// values must not depend on which instantiation its warp runs.
+__device__ __forceinline__ double add_rn(double x, double y) { return __dadd_rn(x, y); }
+__device__ __forceinline__ long long add_rn(long long x, long long y) { return x + y; }
+
+// Sum over the G lanes of a group.
+template <int G, typename T>
+__device__ __forceinline__ T group_sum(T v) {
+#pragma unroll
+  for (int d = G / 2; d > 0; d >>= 1) v = add_rn(v, __shfl_xor_sync(0xffffffffu, v, d, G));
+  return v;
+}
+
+// QR of the group's [At | e_E] (m rows, nj columns of At), back substitution
+// and the column's outputs.  All groups of the warp run it together: `steps` is
+// the group's own min(nj, m), `most` the largest in the warp.  RP rows per
+// lane.  Returns true for a zero / non-finite pivot.
+template <typename T, typename S, int RP, int NJU>
+__device__ __forceinline__ bool rows_qr_solve(const SmallArgs& a, const GroupSmem<T, S>& gs, int lane, int k, int cs,
+                                              int nj, int m, int steps, int most) {
+  constexpr int G = S::G, NC = NJU + 1;  // columns used: NJU of At, then e_E
+  T r[RP][NC];
+#pragma unroll
+  for (int i = 0; i < RP; ++i) {
+    const int row = lane + G * i;
+    const bool in = row < m;
+#pragma unroll
+    for (int c = 0; c < NJU; ++c) r[i][c] = in ? gs.At[row * S::LD + c] : T(0);
+    r[i][NJU] = in ? gs.At[row * S::LD + S::NJ] : T(0);
+  }
+  bool sing = m < nj;
+#pragma unroll
+  for (int c = 0; c < NJU; ++c) {
+    if (c >= most) break;
+    const int ic = c / G, lc = c % G;  // row c: r[ic] of lane lc
+    const bool act = c < steps;
+    // norm of rows >= c
+    T p0 = lane >= lc ? r[ic][c] * r[ic][c] : T(0), p1 = T(0);
+#pragma unroll
+    for (int i = ic + 1; i < RP; ++i) {
+      if ((i - ic) & 1) p1 = fma(r[i][c], r[i][c], p1);
+      else p0 = fma(r[i][c], r[i][c], p0);
+    }
+    const T nrm2 = group_sum<G>(add_rn(p0, p1));
+    const T x0 = __shfl_sync(0xffffffffu, r[ic][c], lc, G);
+    const T nrm = sqrt(nrm2);
+    T alpha = T(0), beta = T(0);
+    if (act) {
+      if (nrm > T(0)) {
+        alpha = (x0 > T(0)) ? -nrm : nrm;
+        beta = T(1) / (nrm * (nrm + fabs(x0)));  // 2 / (v^T v)
+      } else {
+        sing = true;
+      }
+    }
+    // v: rows > c as they are, x0 - alpha at row c, nothing above
+    const T vc = lane > lc ? r[ic][c] : (lane == lc ? x0 - alpha : T(0));
+    T w[NC];
+#pragma unroll
+    for (int j = c + 1; j < NC; ++j) {
+      w[j] = vc * r[ic][j];
+#pragma unroll
+      for (int i = ic + 1; i < RP; ++i) w[j] = fma(r[i][c], r[i][j], w[j]);
+    }
+#pragma unroll
+    for (int j = c + 1; j < NC; ++j) w[j] = group_sum<G>(w[j]) * beta;
+#pragma unroll
+    for (int j = c + 1; j < NC; ++j) {
+      r[ic][j] -= w[j] * vc;
+#pragma unroll
+      for (int i = ic + 1; i < RP; ++i) r[i][j] -= w[j] * r[i][c];
+    }
+    if (act && lane == lc) r[ic][c] = alpha;
+  }
+  // ||(Q^T e_E)[nj:]||^2
+  T res2 = T(0);
+#pragma unroll
+  for (int i = 0; i < RP; ++i)
+    if (lane + G * i >= nj) res2 = fma(r[i][NJU], r[i][NJU], res2);
+  if (a.colres) {
+    res2 = group_sum<G>(res2);
+    if (lane == 0 && nj > 0) a.colres[k - a.col_start] = sqrt((double)res2);
+  }
+  // R x = y: the lane that holds row c forms x_c, the lanes above subtract its column
+#pragma unroll
+  for (int c = NJU - 1; c >= 0; --c) {
+    const int ic = c / G, lc = c % G;
+    T x = T(0);
+    if (c < nj && lane == lc) {
+      const T d = r[ic][c];
+      if (!(d != T(0)) || !isfinite((double)d)) sing = true;
+      x = r[ic][NJU] * (T(1) / d);
+      a.mval[cs + c] = (double)x;
+    }
+    x = __shfl_sync(0xffffffffu, x, lc, G);
+    if (c < nj) {
+#pragma unroll
+      for (int i = 0; i < ic; ++i) r[i][NJU] -= r[i][c] * x;
+      if (lane < lc) r[ic][NJU] -= r[ic][c] * x;
+    }
+  }
+  return sing;
+}
+
+// One column per group of the warp (k < 0: none).  The candidates are t = lane
+// + G i, i < PER.
+template <typename T, typename S, int PER>
+__device__ __forceinline__ int rows_column(const SmallArgs& a, GroupSmem<T, S>& gs, int k, int cs, int nj, int cand,
+                                           int lane, int max_ni, bool* sing) {
+  constexpr int G = S::G;
+  unsigned key[PER], row[PER];
+  T val[PER];
+  int jof[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int t = lane + G * i;
+    int j = 0;
+#pragma unroll
+    for (int q = 1; q < S::NJ; ++q) j += (q < nj && t >= gs.cb[q]) ? 1 : 0;
+    jof[i] = j;
+    row[i] = kPad;
+    val[i] = T(0);
+    if (t < cand) {
+      const int src = gs.base[j] + t;
+      row[i] = (unsigned)__ldg(a.idx + src);
+      val[i] = (T)__ldg(a.val + src);
+    }
+    key[i] = row[i];
+  }
+  rows_sort<G, PER>(key, lane);
+  // distinct rows, in order
+  const unsigned prev = __shfl_up_sync(0xffffffffu, key[PER - 1], 1, G);
+  unsigned first = 0;
+  int cnt = 0;
+#pragma unroll
+  for (int s = 0; s < PER; ++s) {
+    const unsigned before = (s == 0) ? prev : key[s - 1];
+    const bool f = key[s] != kPad && ((s == 0 && lane == 0) || before != key[s]);
+    first |= (f ? 1u : 0u) << s;
+    cnt += f ? 1 : 0;
+  }
+  int inc = cnt;
+#pragma unroll
+  for (int d = 1; d < G; d <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, inc, d, G);
+    if (lane >= d) inc += t;
+  }
+  const int m = __shfl_sync(0xffffffffu, inc, G - 1, G);
+  const bool fits = m <= max_ni;
+  const int mm = fits ? m : 0, njm = fits ? nj : 0;
+  if (fits) {
+    int pos = inc - cnt;
+#pragma unroll
+    for (int s = 0; s < PER; ++s)
+      if (first >> s & 1u) gs.rows[pos++] = key[s];
+    for (int i = lane; i < mm * S::LD; i += G) gs.At[i] = T(0);
+  }
+  if (lane == 0) gs.E = -1;
+  __syncwarp();
+  // rank of a row in I_k
+  auto rank = [&](unsigned rw) {
+    int lo = 0;
+#pragma unroll
+    for (int step = 32; step > 0; step >>= 1)
+      if (step < S::RMAX && lo + step < mm && gs.rows[lo + step] <= rw) lo += step;
+    return lo;
+  };
+  if (fits) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (row[i] != kPad) {
+        const int p = rank(row[i]);
+        gs.At[p * S::LD + jof[i]] = val[i];
+        if (row[i] == (unsigned)k) gs.E = p;
+      }
+  }
+  __syncwarp();
+  if (lane == 0 && fits && gs.E >= 0) gs.At[gs.E * S::LD + S::NJ] = T(1);
+  __syncwarp();
+  const int steps = min(njm, mm);
+  const int most = __reduce_max_sync(0xffffffffu, steps);
+  const int rows = __reduce_max_sync(0xffffffffu, mm);
+  const int wide = __reduce_max_sync(0xffffffffu, njm);
+  // rows per lane and columns by what the warp's largest column needs
+  constexpr int RP = (S::RMAX + G - 1) / G;
+  bool sg;
+  if constexpr (S::NJ == 7) {
+    if (rows <= 16 && wide <= 5) sg = rows_qr_solve<T, S, 4, 5>(a, gs, lane, k, cs, njm, mm, steps, most);
+    else sg = rows_qr_solve<T, S, RP, 7>(a, gs, lane, k, cs, njm, mm, steps, most);
+  } else if constexpr (S::NJ == 11) {
+    if (wide <= 9) sg = rows_qr_solve<T, S, RP, 9>(a, gs, lane, k, cs, njm, mm, steps, most);
+    else sg = rows_qr_solve<T, S, RP, S::NJ>(a, gs, lane, k, cs, njm, mm, steps, most);
+  } else {
+    sg = rows_qr_solve<T, S, RP, S::NJ>(a, gs, lane, k, cs, njm, mm, steps, most);
+  }
+  __syncwarp();
+  *sing = fits && nj > 0 && sg;
+  return fits ? m : -1;
+}
+
+template <typename T, typename S>
+__global__ void __launch_bounds__(GR_BLOCK) k_spai_rows(GroupArgs ga) {
+  extern __shared__ __align__(16) unsigned char rows_raw[];
+  const SmallArgs& a = ga.a;
+  constexpr int G = S::G;
+  const int lane = threadIdx.x & (G - 1), wl = threadIdx.x & 31;
+  const int g = wl / G;
+  GroupSmem<T, S>& gs = reinterpret_cast<GroupSmem<T, S>*>(rows_raw)[threadIdx.x / G];
+  const int warp = (blockIdx.x * GR_BLOCK + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * GR_BLOCK) >> 5;
+  int my_max_ni = 0, my_max_nj = 0, my_cols = 0, my_sing = 0;
+
+  // the next size for a column this one does not take (lane 0 of its group)
+  auto pass_on = [&](int k, int nj, long long cand) {
+    if (ga.mid_list && S::NJ < GroupB::NJ && nj <= GroupB::NJ && cand <= GroupB::CMAX)
+      ga.mid_list[atomicAdd(&a.stats[ST_MID_COUNT], 1)] = k;
+    else if (ga.mid_list && S::NJ < GroupC::NJ && nj <= GroupC::NJ && cand <= GroupC::CMAX)
+      ga.wide_list[atomicAdd(&a.stats[ST_WIDE_COUNT], 1)] = k;
+    else
+      queue_big(a, k, nj, cand * (nj + 1));
+  };
+
+  auto process = [&](int k) {  // k < 0: this group has no column this time
+    int cs = 0, nj = 0;
+    if (k >= 0) {
+      cs = __ldg(a.ptr + k);
+      nj = __ldg(a.ptr + k + 1) - cs;
+    }
+    my_max_nj = max(my_max_nj, nj);
+    if (k >= 0 && nj == 0) {
+      if (lane == 0 && a.colres) a.colres[k - a.col_start] = 1.0;
+      ++my_cols;
+    }
+    long long cand = 0;
+    if (__any_sync(0xffffffffu, nj > S::NJ)) {
+      // a column too wide for this size: its candidates, as a bound of its block
+      if (nj > S::NJ)
+        for (int t = lane; t < nj; t += G) {
+          const int j = __ldg(a.idx + cs + t);
+          cand += __ldg(a.ptr + j + 1) - __ldg(a.ptr + j);
+        }
+      cand = group_sum<G>(cand);
+      if (nj > S::NJ) {
+        if (lane == 0) pass_on(k, nj, cand);
+        nj = 0;
+      }
+    }
+    // candidate offsets of the J columns
+    int c2 = 0;
+#pragma unroll
+    for (int j0 = 0; j0 < S::NJ; j0 += G) {
+      const int j = j0 + lane;
+      int b = 0, l = 0;
+      if (j < nj) {
+        const int col = __ldg(a.idx + cs + j);
+        b = __ldg(a.ptr + col);
+        l = __ldg(a.ptr + col + 1) - b;
+      }
+      int inc = l;
+#pragma unroll
+      for (int d = 1; d < G; d <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, d, G);
+        if (lane >= d) inc += t;
+      }
+      if (j < S::NJ) {
+        gs.cb[j] = c2 + inc - l;
+        gs.base[j] = b - (c2 + inc - l);
+      }
+      c2 += __shfl_sync(0xffffffffu, inc, G - 1, G);
+    }
+    if (c2 > S::CMAX) {
+      if (lane == 0) pass_on(k, nj, c2);
+      nj = 0;
+      c2 = 0;
+    }
+    __syncwarp();
+    bool sing = false;
+    const int most = __reduce_max_sync(0xffffffffu, c2);
+    if (most == 0) return;
+    // the sort's size by what the warp's largest column needs
+    const int m = (most <= S::CMAX / 2)
+                      ? rows_column<T, S, S::PER / 2>(a, gs, k, cs, nj, c2, lane, min(a.max_ni, S::RMAX), &sing)
+                      : rows_column<T, S, S::PER>(a, gs, k, cs, nj, c2, lane, min(a.max_ni, S::RMAX), &sing);
+    if (nj > 0) {
+      if (m < 0) {
+        if (lane == 0) pass_on(k, nj, c2);
+      } else {
+        my_max_ni = max(my_max_ni, m);
+        ++my_cols;
+      }
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, sing);
+    if (lane == 0 && ((any >> (g * G)) & ((1ull << G) - 1u))) ++my_sing;
+  };
+
+  if (ga.in) {
+    const int count = a.stats[ga.in_count];
+    for (int q = warp * S::GPW; q < count; q += nwarps * S::GPW) process(q + g < count ? ga.in[q + g] : -1);
+  } else if (a.schedule == DCU_SCHED_BALANCED_COLUMNS) {
+    // balanced_columns: one sweep of the whole range by all warps, so that
+    // they work in one window of A (see k_spai_small)
+    for (int k = a.col_start + warp * S::GPW; k < a.col_end; k += nwarps * S::GPW)
+      process(k + g < a.col_end ? k + g : -1);
+  } else {
+    // nnz-balanced chunks pulled from the queue, a chunk to a warp
+    for (;;) {
+      int ch = 0;
+      if (wl == 0) ch = atomicAdd(&a.stats[ST_DYN_HEAD], 1);
+      ch = __shfl_sync(0xffffffffu, ch, 0);
+      if (ch >= a.nchunks) break;
+      const int e = a.chunks[ch + 1];
+      for (int k = a.chunks[ch]; k < e; k += S::GPW) process(k + g < e ? k + g : -1);
+    }
+  }
+  if (lane == 0) {
+    atomicMax(&a.stats[ST_MAXNI], my_max_ni);
+    atomicMax(&a.stats[ST_MAXNJ], my_max_nj);
+    if (my_cols) atomicAdd(&a.stats[ST_SMALL_COLS], my_cols);
+    if (my_sing) atomicAdd(&a.stats[ST_SINGULAR], my_sing);
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Thread per column: the batched least-squares path of the mixed forms.
@@ -1334,6 +1752,69 @@ int run_small(Ctx* c, SmallArgs a, int) {
   return DCU_OK;
 }
 
+// FP64 build over the column range (or over the `in` list): the three sizes of
+// the group kernel, each over what the one before passed on.
+template <typename T, typename S>
+int launch_rows(Ctx* c, GroupArgs ga) {
+  auto kernel = k_spai_rows<T, S>;
+  const size_t smem = sizeof(GroupSmem<T, S>) * (GR_BLOCK / S::G);
+  DCU_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GR_BLOCK, smem) != cudaSuccess || per_sm < 1) {
+    cudaGetLastError();
+    per_sm = 1;
+  }
+  const int grid = c->sms * per_sm;
+  SmallArgs& a = ga.a;
+  if (!ga.in && a.schedule == DCU_SCHED_BALANCED_NNZ) {
+    const int nchunks = grid * (GR_BLOCK / 32) * 4;
+    DCU_TRY(ensure(c, B_CHUNKS, sizeof(int) * (size_t)(nchunks + 1)));
+    int* bounds = bp<int>(c, B_CHUNKS);
+    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds);
+    DCU_LAUNCHED(c, "k_nnz_chunks");
+    a.chunks = bounds;
+    a.nchunks = nchunks;
+  }
+  kernel<<<grid, GR_BLOCK, smem, c->stream>>>(ga);
+  DCU_LAUNCHED(c, "k_spai_rows");
+  return DCU_OK;
+}
+
+// First size: the range, or the columns the thread kernel handed over.  With
+// a tuned |I| limit the columns above it go to the CTA kernel.
+template <typename T>
+int run_rows(Ctx* c, const SmallArgs& sa) {
+  GroupArgs ga{};
+  ga.a = sa;
+  ga.in = sa.list;
+  ga.in_count = ST_FB_COUNT;
+  if (sa.max_ni >= SG_MMAX) {
+    const size_t n = (size_t)std::max(1, sa.col_end - sa.col_start);
+    DCU_TRY(ensure(c, B_MIDLIST, sizeof(int) * 2 * n));
+    ga.mid_list = bp<int>(c, B_MIDLIST);
+    ga.wide_list = ga.mid_list + n;
+  }
+  return launch_rows<T, GroupA>(c, ga);
+}
+
+// The second and third size, over what the first (and second) passed on.
+template <typename T>
+int run_rows_rest(Ctx* c, const SmallArgs& sa, int mid) {
+  GroupArgs ga{};
+  ga.a = sa;
+  ga.mid_list = bp<int>(c, B_MIDLIST);
+  ga.wide_list = ga.mid_list + std::max(1, sa.col_end - sa.col_start);
+  ga.a.max_ni = INT_MAX;
+  if (mid > 0) {
+    ga.in = ga.mid_list;
+    ga.in_count = ST_MID_COUNT;
+    DCU_TRY((launch_rows<T, GroupB>(c, ga)));
+  }
+  ga.in = ga.wide_list;
+  ga.in_count = ST_WIDE_COUNT;
+  return launch_rows<T, GroupC>(c, ga);
+}
+
 template <typename T, int MODE>
 int run_large(Ctx* c, LargeArgs& a, int nbig, int cta_max_area = 0) {
   const size_t fixed = ((sizeof(LargeSmem<T>) + 15) / 16) * 16 + LG_STAGE_BYTES;
@@ -1526,6 +2007,8 @@ int build_launch(Ctx* c, int n, const int* ptr, const int* idx, const double* va
     na.tau = sizeof(T) == sizeof(float) ? 1e-3 : 1e-8;
     J->fb_list = na.fb_list;
     DCU_TRY(run_ne<T>(c, na));
+  } else if constexpr (std::is_same<T, double>::value) {
+    DCU_TRY(run_rows<T>(c, P.sa));
   } else {
     DCU_TRY((run_small<T, MODE_BUILD>(c, P.sa, P.grid)));
   }
@@ -1542,10 +2025,16 @@ int build_finish(Ctx* c, int n, const int* ptr, const int* idx, const double* va
     if (st[ST_FB_COUNT] > 0) {
       P.sa.list = J->fb_list;
       J->finish_launched = true;
-      DCU_TRY((run_small<T, MODE_BUILD>(c, P.sa, P.grid)));
+      if constexpr (std::is_same<T, double>::value) DCU_TRY(run_rows<T>(c, P.sa));
+      else DCU_TRY((run_small<T, MODE_BUILD>(c, P.sa, P.grid)));
     }
   }
   DCU_TRY(read_stats(c, st));
+  if (st[ST_MID_COUNT] + st[ST_WIDE_COUNT] > 0) {
+    J->finish_launched = true;
+    DCU_TRY(run_rows_rest<double>(c, P.sa, st[ST_MID_COUNT]));
+    DCU_TRY(read_stats(c, st));
+  }
   const int nbig = st[ST_BIG_COUNT];
   if (nbig > 0) {
     if (st[ST_BIG_MAXNJ] > LG_NJ_MAX)
@@ -1585,16 +2074,8 @@ int build_finish(Ctx* c, int n, const int* ptr, const int* idx, const double* va
 
 }  // namespace
 
-int spai_default_units(Ctx* c) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_spai_small<double, MODE_BUILD>, SG_BLOCK, 0) !=
-          cudaSuccess ||
-      per_sm < 1) {
-    cudaGetLastError();
-    per_sm = 1;
-  }
-  return c->sms * per_sm * (SG_BLOCK / GL);
-}
+// One unit per resident 16-lane group of k_spai_small (12 blocks per SM).
+int spai_default_units(Ctx* c) { return c->sms * 12 * (SG_BLOCK / GL); }
 
 BuildJob::BuildJob() : impl(new BuildJobImpl) {}
 BuildJob::~BuildJob() { delete impl; }
