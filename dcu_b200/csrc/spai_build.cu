@@ -466,7 +466,7 @@ __global__ void __launch_bounds__(SG_BLOCK, 12) k_spai_small(SmallArgs a) {
 // columns run in lockstep through one unrolled step loop.  (Two lanes per
 // column of [At | e_E], the layout of k_spai_small, leaves the lanes of finished
 // columns idle and re-reads v from shared memory: 4.6 ms at 128^3 on one B200,
-// this one 1.1 ms.)  I_k: the candidate rows of A(:, J) are sorted across the
+// this one 1.5 ms.)  I_k: the candidate rows of A(:, J) are sorted across the
 // group (bitonic network in registers) and ranked; At is scattered into shared
 // memory and read back by rows.
 //
@@ -504,14 +504,14 @@ struct GroupArgs {
 template <typename T, typename S>
 struct GroupSmemRaw {
   T At[S::RMAX * S::LD];
-  unsigned rows[S::RMAX];   // I_k
+  unsigned rows[S::RMAX];   // I_k (or the candidates' ranks, a byte each)
   int base[S::NJ + 1];      // start of J column j in A's arrays, minus its first candidate
   int cb[S::NJ + 1];        // first candidate of J column j
   int E;
 };
 // padded so that the groups of a warp start 8 banks apart
 template <typename T, typename S>
-struct alignas(8) GroupSmem : GroupSmemRaw<T, S> {
+struct alignas(16) GroupSmem : GroupSmemRaw<T, S> {
   static constexpr int words = (int)(sizeof(GroupSmemRaw<T, S>) / 4);
   static constexpr int more = (40 - words % 32) % 32;
   int pad[more ? more : 32];
@@ -652,11 +652,30 @@ __device__ __forceinline__ bool rows_qr_solve(const SmallArgs& a, const GroupSme
   return sing;
 }
 
-// One column per group of the warp (k < 0: none).  The candidates are t = lane
-// + G i, i < PER.
+// QR and solution of the groups' columns once At holds them, on the rows and
+// columns that the warp's largest column needs.  mm = 0 for a group without one.
+template <typename T, typename S>
+__device__ __forceinline__ bool rows_solve(const SmallArgs& a, const GroupSmem<T, S>& gs, int k, int cs, int njm, int mm,
+                                           int lane) {
+  const int steps = min(njm, mm);
+  const int most = __reduce_max_sync(0xffffffffu, steps);
+  const int rows = __reduce_max_sync(0xffffffffu, mm);
+  const int wide = __reduce_max_sync(0xffffffffu, njm);
+  constexpr int RP = (S::RMAX + S::G - 1) / S::G;
+  if constexpr (S::NJ == 7) {
+    if (rows <= 16 && wide <= 5) return rows_qr_solve<T, S, 4, 5>(a, gs, lane, k, cs, njm, mm, steps, most);
+  } else if constexpr (S::NJ == 11) {
+    if (wide <= 9) return rows_qr_solve<T, S, RP, 9>(a, gs, lane, k, cs, njm, mm, steps, most);
+  }
+  return rows_qr_solve<T, S, RP, S::NJ>(a, gs, lane, k, cs, njm, mm, steps, most);
+}
+
+// I_k and At of one column per group of the warp (k < 0: none) in shared
+// memory; returns |I_k|, and leaves At alone where it exceeds max_ni.  The
+// candidates are t = lane + G i, i < PER.
 template <typename T, typename S, int PER>
-__device__ __forceinline__ int rows_column(const SmallArgs& a, GroupSmem<T, S>& gs, int k, int cs, int nj, int cand,
-                                           int lane, int max_ni, bool* sing) {
+__device__ __forceinline__ int rows_stage(const SmallArgs& a, GroupSmem<T, S>& gs, int k, int nj, int cand, int lane,
+                                          int max_ni) {
   constexpr int G = S::G;
   unsigned key[PER], row[PER];
   T val[PER];
@@ -697,7 +716,7 @@ __device__ __forceinline__ int rows_column(const SmallArgs& a, GroupSmem<T, S>& 
   }
   const int m = __shfl_sync(0xffffffffu, inc, G - 1, G);
   const bool fits = m <= max_ni;
-  const int mm = fits ? m : 0, njm = fits ? nj : 0;
+  const int mm = fits ? m : 0;
   if (fits) {
     int pos = inc - cnt;
 #pragma unroll
@@ -727,29 +746,108 @@ __device__ __forceinline__ int rows_column(const SmallArgs& a, GroupSmem<T, S>& 
   __syncwarp();
   if (lane == 0 && fits && gs.E >= 0) gs.At[gs.E * S::LD + S::NJ] = T(1);
   __syncwarp();
-  const int steps = min(njm, mm);
-  const int most = __reduce_max_sync(0xffffffffu, steps);
-  const int rows = __reduce_max_sync(0xffffffffu, mm);
-  const int wide = __reduce_max_sync(0xffffffffu, njm);
-  // rows per lane and columns by what the warp's largest column needs
-  constexpr int RP = (S::RMAX + G - 1) / G;
-  bool sg;
-  if constexpr (S::NJ == 7) {
-    if (rows <= 16 && wide <= 5) sg = rows_qr_solve<T, S, 4, 5>(a, gs, lane, k, cs, njm, mm, steps, most);
-    else sg = rows_qr_solve<T, S, RP, 7>(a, gs, lane, k, cs, njm, mm, steps, most);
-  } else if constexpr (S::NJ == 11) {
-    if (wide <= 9) sg = rows_qr_solve<T, S, RP, 9>(a, gs, lane, k, cs, njm, mm, steps, most);
-    else sg = rows_qr_solve<T, S, RP, S::NJ>(a, gs, lane, k, cs, njm, mm, steps, most);
-  } else {
-    sg = rows_qr_solve<T, S, RP, S::NJ>(a, gs, lane, k, cs, njm, mm, steps, most);
+  return m;
+}
+
+// Four lanes, columns of at most 8 ascending rows (every stencil): lane l owns
+// J columns 2 l and 2 l + 1, so its candidates are static (no search for their
+// column, loads at fixed offsets), the eight sorted lists need only the last
+// three merge phases of the network (alternating directions come from
+// complementing the keys), and the key carries the candidate, whose rank comes
+// back through one byte of shared memory.  Returns |I_k| as rows_stage.
+template <typename T, typename S>
+__device__ __forceinline__ int rows_stage_lists(GroupSmem<T, S>& gs, int k, const int (&row)[16], const T (&val)[16],
+                                                int lane, int max_ni) {
+  static_assert(S::G == 4 && S::PER == 16, "eight lists of eight");
+  constexpr int G = 4;
+  unsigned key[16];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {  // the second list descending
+    key[q] = row[q] >= 0 ? ((unsigned)row[q] << 6) | (unsigned)(lane * 16 + q) : kPad;
+    key[15 - q] = row[8 + q] >= 0 ? ((unsigned)row[8 + q] << 6) | (unsigned)(lane * 16 + 8 + q) : kPad;
+  }
+  auto flip = [&](unsigned mask) {
+#pragma unroll
+    for (int s = 0; s < 16; ++s) key[s] ^= mask;
+  };
+  auto merge = [&]() {  // a bitonic run of 16 within the lane, ascending
+#pragma unroll
+    for (int jj = 8; jj > 0; jj >>= 1)
+#pragma unroll
+      for (int s = 0; s < 16; ++s)
+        if (!(s & jj)) {
+          const unsigned x = key[s], y = key[s | jj];
+          key[s] = min(x, y);
+          key[s | jj] = max(x, y);
+        }
+  };
+  auto cross = [&](int lx) {
+    const bool low = (lane & lx) == 0;
+#pragma unroll
+    for (int s = 0; s < 16; ++s) {
+      const unsigned other = __shfl_xor_sync(0xffffffffu, key[s], lx, G);
+      key[s] = low ? min(key[s], other) : max(key[s], other);
+    }
+  };
+  const unsigned m16 = (lane & 1) ? 0xffffffffu : 0u, m32 = (lane & 2) ? 0xffffffffu : 0u;
+  flip(m16);
+  merge();
+  flip(m16 ^ m32);
+  cross(1);
+  merge();
+  flip(m32);
+  cross(2);
+  cross(1);
+  merge();
+  const unsigned prev = __shfl_up_sync(0xffffffffu, key[15], 1, G);
+  unsigned first = 0;
+#pragma unroll
+  for (int s = 0; s < 16; ++s) {
+    const unsigned before = s == 0 ? prev : key[s - 1];
+    const bool f = key[s] != kPad && ((s == 0 && lane == 0) || (before >> 6) != (key[s] >> 6));
+    first |= (f ? 1u : 0u) << s;
+  }
+  const int cnt = __popc(first);
+  int inc = cnt;
+#pragma unroll
+  for (int d = 1; d < G; d <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, inc, d, G);
+    if (lane >= d) inc += t;
+  }
+  const int m = __shfl_sync(0xffffffffu, inc, G - 1, G);
+  const bool fits = m <= max_ni;
+  const int mm = fits ? m : 0;
+  unsigned char* rank = reinterpret_cast<unsigned char*>(gs.rows);
+  if (lane == 0) gs.E = -1;
+  if (fits) {
+    double2* z = reinterpret_cast<double2*>(gs.At);
+    for (int i = lane; 2 * i < mm * S::LD; i += G) z[i] = make_double2(0.0, 0.0);
+    const int before = inc - cnt - 1;
+#pragma unroll
+    for (int s = 0; s < 16; ++s)
+      if (key[s] != kPad) rank[key[s] & 63u] = (unsigned char)(before + __popc(first & ((2u << s) - 1u)));
   }
   __syncwarp();
-  *sing = fits && nj > 0 && sg;
-  return fits ? m : -1;
+  if (fits) {
+    const uint4 r4 = *reinterpret_cast<const uint4*>(rank + lane * 16);
+    const unsigned rw[4] = {r4.x, r4.y, r4.z, r4.w};
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+      if (row[e] >= 0) {
+        const int p = (int)(rw[e >> 2] >> (8 * (e & 3)) & 255u);
+        gs.At[p * S::LD + 2 * lane + (e >> 3)] = val[e];
+        if (row[e] == k) gs.E = p;
+      }
+  }
+  __syncwarp();
+  if (lane == 0 && fits && gs.E >= 0) gs.At[gs.E * S::LD + S::NJ] = T(1);
+  __syncwarp();
+  return m;
 }
 
 template <typename T, typename S>
-__global__ void __launch_bounds__(GR_BLOCK) k_spai_rows(GroupArgs ga) {
+// (6 blocks an SM for the first two sizes without spilling in the steps)
+__global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(GroupArgs ga) {
   extern __shared__ __align__(16) unsigned char rows_raw[];
   const SmallArgs& a = ga.a;
   constexpr int G = S::G;
@@ -795,72 +893,114 @@ __global__ void __launch_bounds__(GR_BLOCK) k_spai_rows(GroupArgs ga) {
         nj = 0;
       }
     }
-    // candidate offsets of the J columns
-    int c2 = 0;
+    const int max_ni = min(a.max_ni, S::RMAX);
+    int m = 0, c2 = 0;
+    bool staged = false;
+    if constexpr (S::G == 4) {
+      int b0 = 0, b1 = 0, l0 = 0, l1 = 0;
+      if (2 * lane < nj) {
+        const int j = __ldg(a.idx + cs + 2 * lane);
+        b0 = __ldg(a.ptr + j);
+        l0 = __ldg(a.ptr + j + 1) - b0;
+      }
+      if (2 * lane + 1 < nj) {
+        const int j = __ldg(a.idx + cs + 2 * lane + 1);
+        b1 = __ldg(a.ptr + j);
+        l1 = __ldg(a.ptr + j + 1) - b1;
+      }
+      if (!__any_sync(0xffffffffu, l0 > 8 || l1 > 8)) {
+        int row[16];
+        T val[16];
+        bool up = true;
 #pragma unroll
-    for (int j0 = 0; j0 < S::NJ; j0 += G) {
-      const int j = j0 + lane;
-      int b = 0, l = 0;
-      if (j < nj) {
-        const int col = __ldg(a.idx + cs + j);
-        b = __ldg(a.ptr + col);
-        l = __ldg(a.ptr + col + 1) - b;
-      }
-      int inc = l;
+        for (int q = 0; q < 8; ++q) {
+          row[q] = q < l0 ? __ldg(a.idx + b0 + q) : -1;
+          row[8 + q] = q < l1 ? __ldg(a.idx + b1 + q) : -1;
+          val[q] = q < l0 ? (T)__ldg(a.val + b0 + q) : T(0);
+          val[8 + q] = q < l1 ? (T)__ldg(a.val + b1 + q) : T(0);
+        }
 #pragma unroll
-      for (int d = 1; d < G; d <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, inc, d, G);
-        if (lane >= d) inc += t;
+        for (int q = 1; q < 8; ++q) up = up && (q >= l0 || row[q] > row[q - 1]) && (q >= l1 || row[8 + q] > row[7 + q]);
+        if (__all_sync(0xffffffffu, up)) {
+          m = rows_stage_lists<T, S>(gs, k, row, val, lane, max_ni);
+          c2 = l0 + l1;
+          c2 += __shfl_xor_sync(0xffffffffu, c2, 1);
+          c2 += __shfl_xor_sync(0xffffffffu, c2, 2);
+          staged = true;
+        }
       }
-      if (j < S::NJ) {
-        gs.cb[j] = c2 + inc - l;
-        gs.base[j] = b - (c2 + inc - l);
+    }
+    if (!staged) {
+      // candidate offsets of the J columns
+#pragma unroll
+      for (int j0 = 0; j0 < S::NJ; j0 += G) {
+        const int j = j0 + lane;
+        int b = 0, l = 0;
+        if (j < nj) {
+          const int col = __ldg(a.idx + cs + j);
+          b = __ldg(a.ptr + col);
+          l = __ldg(a.ptr + col + 1) - b;
+        }
+        int inc = l;
+#pragma unroll
+        for (int d = 1; d < G; d <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, inc, d, G);
+          if (lane >= d) inc += t;
+        }
+        if (j < S::NJ) {
+          gs.cb[j] = c2 + inc - l;
+          gs.base[j] = b - (c2 + inc - l);
+        }
+        c2 += __shfl_sync(0xffffffffu, inc, G - 1, G);
       }
-      c2 += __shfl_sync(0xffffffffu, inc, G - 1, G);
-    }
-    if (c2 > S::CMAX) {
-      if (lane == 0) pass_on(k, nj, c2);
-      nj = 0;
-      c2 = 0;
-    }
-    __syncwarp();
-    bool sing = false;
-    const int most = __reduce_max_sync(0xffffffffu, c2);
-    if (most == 0) return;
-    // the sort's size by what the warp's largest column needs
-    const int m = (most <= S::CMAX / 2)
-                      ? rows_column<T, S, S::PER / 2>(a, gs, k, cs, nj, c2, lane, min(a.max_ni, S::RMAX), &sing)
-                      : rows_column<T, S, S::PER>(a, gs, k, cs, nj, c2, lane, min(a.max_ni, S::RMAX), &sing);
-    if (nj > 0) {
-      if (m < 0) {
+      if (c2 > S::CMAX) {
         if (lane == 0) pass_on(k, nj, c2);
+        nj = 0;
+        c2 = 0;
+      }
+      __syncwarp();
+      // the sort's size by what the warp's largest column needs
+      const int most = __reduce_max_sync(0xffffffffu, c2);
+      if (most > S::CMAX / 2) m = rows_stage<T, S, S::PER>(a, gs, k, nj, c2, lane, max_ni);
+      else if (most > 0) m = rows_stage<T, S, S::PER / 2>(a, gs, k, nj, c2, lane, max_ni);
+    }
+    if (nj > 0) {
+      if (m > max_ni) {
+        if (lane == 0) pass_on(k, nj, c2);
+        nj = 0;
+        m = 0;
       } else {
         my_max_ni = max(my_max_ni, m);
         ++my_cols;
       }
     }
+    if (!__any_sync(0xffffffffu, nj > 0)) return;
+    const bool sing = rows_solve<T, S>(a, gs, k, cs, nj, nj > 0 ? m : 0, lane) && nj > 0;
     const unsigned any = __ballot_sync(0xffffffffu, sing);
     if (lane == 0 && ((any >> (g * G)) & ((1ull << G) - 1u))) ++my_sing;
+    __syncwarp();
   };
 
-  if (ga.in) {
-    const int count = a.stats[ga.in_count];
-    for (int q = warp * S::GPW; q < count; q += nwarps * S::GPW) process(q + g < count ? ga.in[q + g] : -1);
-  } else if (a.schedule == DCU_SCHED_BALANCED_COLUMNS) {
-    // balanced_columns: one sweep of the whole range by all warps, so that
-    // they work in one window of A (see k_spai_small)
-    for (int k = a.col_start + warp * S::GPW; k < a.col_end; k += nwarps * S::GPW)
-      process(k + g < a.col_end ? k + g : -1);
-  } else {
-    // nnz-balanced chunks pulled from the queue, a chunk to a warp
-    for (;;) {
+  // The columns: a list, the whole range in one sweep by all warps (so that
+  // they work in one window of A, see k_spai_small), or nnz-balanced chunks
+  // pulled from the queue, a chunk to a warp.
+  const bool chunked = !ga.in && a.schedule != DCU_SCHED_BALANCED_COLUMNS;
+  const int step = (chunked ? 1 : nwarps) * S::GPW;
+  int pos = chunked ? 0 : warp * S::GPW + (ga.in ? 0 : a.col_start);
+  int end = chunked ? 0 : ga.in ? a.stats[ga.in_count] : a.col_end;
+  for (;;) {
+    if (pos >= end) {
+      if (!chunked) break;
       int ch = 0;
       if (wl == 0) ch = atomicAdd(&a.stats[ST_DYN_HEAD], 1);
       ch = __shfl_sync(0xffffffffu, ch, 0);
       if (ch >= a.nchunks) break;
-      const int e = a.chunks[ch + 1];
-      for (int k = a.chunks[ch]; k < e; k += S::GPW) process(k + g < e ? k + g : -1);
+      pos = a.chunks[ch];
+      end = a.chunks[ch + 1];
+      continue;
     }
+    process(pos + g >= end ? -1 : ga.in ? ga.in[pos + g] : pos + g);
+    pos += step;
   }
   if (lane == 0) {
     atomicMax(&a.stats[ST_MAXNI], my_max_ni);
@@ -1711,8 +1851,9 @@ __global__ void __launch_bounds__(LG_BLOCK) k_hub_solve(HubArgs h, LargeArgs a) 
 
 // nnz-balanced chunk bounds for the dynamic schedule: chunk c starts at the
 // first column whose nnz prefix reaches c/nchunks of the range's nnz.
+// Bounds are rounded up to `grain` columns from the first.
 __global__ void k_nnz_chunks(const int* __restrict__ ptr, int col_start, int col_end, int nchunks,
-                             int* __restrict__ bounds) {
+                             int* __restrict__ bounds, int grain) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c > nchunks) return;
   const long long p0 = ptr[col_start], tot = (long long)ptr[col_end] - p0;
@@ -1725,7 +1866,7 @@ __global__ void k_nnz_chunks(const int* __restrict__ ptr, int col_start, int col
     if ((long long)ptr[mid] < target) lo = mid + 1;
     else hi = mid;
   }
-  bounds[c] = lo;
+  bounds[c] = min(col_end, col_start + (lo - col_start + grain - 1) / grain * grain);
 }
 
 template <typename T, int MODE>
@@ -1742,7 +1883,7 @@ int run_small(Ctx* c, SmallArgs a, int) {
     const int nchunks = ngroups * 4;
     DCU_TRY(ensure(c, B_CHUNKS, sizeof(int) * (size_t)(nchunks + 1)));
     int* bounds = bp<int>(c, B_CHUNKS);
-    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds);
+    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds, 1);
     DCU_LAUNCHED(c, "k_nnz_chunks");
     a.chunks = bounds;
     a.nchunks = nchunks;
@@ -1767,10 +1908,11 @@ int launch_rows(Ctx* c, GroupArgs ga) {
   const int grid = c->sms * per_sm;
   SmallArgs& a = ga.a;
   if (!ga.in && a.schedule == DCU_SCHED_BALANCED_NNZ) {
-    const int nchunks = grid * (GR_BLOCK / 32) * 4;
+    // about 4 steps of a warp to a chunk
+    const int nchunks = std::max(1, std::min(grid * (GR_BLOCK / 32) * 4, (a.col_end - a.col_start) / (4 * S::GPW)));
     DCU_TRY(ensure(c, B_CHUNKS, sizeof(int) * (size_t)(nchunks + 1)));
     int* bounds = bp<int>(c, B_CHUNKS);
-    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds);
+    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds, S::GPW);
     DCU_LAUNCHED(c, "k_nnz_chunks");
     a.chunks = bounds;
     a.nchunks = nchunks;
@@ -1919,7 +2061,7 @@ int run_ne(Ctx* c, NeArgs a) {
     const int nchunks = grid * 8;
     DCU_TRY(ensure(c, B_CHUNKS, sizeof(int) * (size_t)(nchunks + 1)));
     int* bounds = bp<int>(c, B_CHUNKS);
-    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds);
+    k_nnz_chunks<<<(nchunks + 256) / 256, 256, 0, c->stream>>>(a.ptr, a.col_start, a.col_end, nchunks, bounds, 1);
     DCU_LAUNCHED(c, "k_nnz_chunks");
     a.chunks = bounds;
     a.nchunks = nchunks;

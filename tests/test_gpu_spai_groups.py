@@ -88,3 +88,22 @@ def test_mixed_widths_share_warps(ctx):
     A = W.CSC(n, ptr, np.concatenate([cols[c][0] for c in range(n)]).astype(np.int32),
               np.concatenate([cols[c][1] for c in range(n)]))
     check(ctx, A)
+
+
+def test_columns_of_empty_columns(ctx):
+    """J columns without entries: |I| = 0, reported singular, the others unharmed."""
+    n = 40
+    ptr, idx, val = [0], [], []
+    for c in range(n):
+        if c not in (3, 4):                       # columns 3 and 4 are empty
+            rows = [3] if c == 0 else [3, 4] if c == 9 else [c]
+            idx += rows
+            val += [2.0] * len(rows)
+        ptr.append(len(idx))
+    A = W.CSC(n, np.array(ptr, np.int32), np.array(idx, np.int32), np.array(val))
+    # (no oracle here: it does not take |I| = 0.)  A column that holds only its diagonal: m = 1 / 2
+    m, res, info = ctx.build_h(A, precision=N.PREC_FP64)
+    assert info.cols_singular == 2 and info.cols_small == n
+    alone = np.ones(A.nnz, bool)
+    alone[A.ptr[0]:A.ptr[1]] = alone[A.ptr[9]:A.ptr[10]] = False
+    assert np.all(m[alone] == 0.5) and not np.any(np.isfinite(m[~alone]))
