@@ -563,6 +563,499 @@ __global__ void kb_step(BArgs<R> a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// A cluster per system.
+//
+// The kernels above run every system's tiles in each launch: an iteration of
+// the whole batch streams all its vectors through HBM and costs six launches.
+// Here one cluster takes a
+// system through its whole solve before the next one, its rows split over the
+// cluster's CTAs, so that the vectors of the systems in flight stay in L2 (and
+// r*, Az and x, which only their own row reads, in shared memory where they
+// fit); the five steps of an iteration are separated by the cluster's hardware
+// barrier, and a system costs its own iterations, not the batch's.  s and p are
+// not stored: s = r - alpha Ay and p = r + beta q (q = p - omega Ay of the last
+// iteration, published with r) are formed where they are used, by the same
+// operations.  Systems are taken from a queue, the large ones from one end by
+// the even clusters, the small ones from the other by the odd ones, so that
+// large systems do not all share L2 at once.  Each CTA sums the same partials
+// in the same order; a system's result does not depend on the order of the
+// queue.
+// ---------------------------------------------------------------------------
+constexpr int BC_THREADS = 512;   // (1024 hold 64 registers each and spill: 265 -> 340 ms on 512 systems x 8)
+constexpr int BC_MAXC = 16;
+
+struct BCArgs {
+  int count;                // systems of this launch ...
+  const int* order;         // ... by size, descending
+  int* head;                // [0] taken, [1] from the front, [2] from the back
+  const int* sys_off;
+  const long long* off;
+  const int* kd;
+  const int* su;
+  const int* ix;
+  const double* aval;
+  const double* mval;
+  const double* b;
+  double* x;
+  double *r, *q, *y, *ay, *z, *rs, *az;
+  double tol;
+  int tol_mode, maxiter;
+  int cap;                  // doubles of dynamic shared memory
+  int* iters;
+  int* status;
+};
+
+__device__ __forceinline__ unsigned bc_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned bc_size() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned bc_id() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned bc_remote(const void* p, unsigned rank) {
+  unsigned o;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return o;
+}
+__device__ __forceinline__ void bc_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// A row's entries reach the CTA's shared memory a pass ahead of their use
+// (cp.async, each row's copies by the T threads that share it, so a warp waits
+// for its own copies only): a pass then waits for one gather instead of the
+// chain slice offset -> values and columns -> gather.
+constexpr int BC_W = 8;           // entries of a row that are prefetched (the rest are read in place)
+constexpr int BC_LD = BC_W + 1;   // row stride (rows in different banks)
+constexpr int BC_STAGES = 2;
+constexpr int BC_SLICES = 256;    // 32-row slices of one CTA, at most
+
+template <int R>
+struct BCEntries {
+  static constexpr int ROWS = BC_THREADS / (R / vals_per_thread<R>());  // rows of a pass
+  double val[BC_STAGES][ROWS * BC_LD];
+  int col[BC_STAGES][ROWS * BC_LD];
+  int off[BC_SLICES + 1];         // first slot of each of the CTA's slices, from the first one's
+};
+template <int R>
+__host__ __device__ constexpr size_t bc_entry_bytes() {
+  static_assert(sizeof(BCEntries<R>) <= 128 * 1024, "room for the rows' own vectors, and for the entries at all");
+  return (sizeof(BCEntries<R>) + 15) / 16 * 16;
+}
+
+__device__ __forceinline__ void bc_copy8(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" : : "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void bc_copy4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" : : "r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// The rows of one CTA: entries ahead of their use, and their sums.
+template <int R>
+struct BCRows {
+  static constexpr int V = vals_per_thread<R>(), T = R / V, ROWS = BCEntries<R>::ROWS;
+  BCEntries<R>& E;
+  const long long* off;
+  const int* ix;
+  int c0, rows, sl0;
+  long long ob;   // first slot of the CTA's first slice
+
+  __device__ __forceinline__ void prefetch(const double* val, int pass) const {
+    const int jr = threadIdx.x / T, j = pass * ROWS + jr;
+    if (j < rows) {
+      const int row = c0 + j, sl = (row >> 5) - sl0;
+      const int o = E.off[sl], w = min(BC_W, (E.off[sl + 1] - o) >> 5);
+      const long long at = ob + o + (row & 31);
+      double* dv = &E.val[pass % BC_STAGES][jr * BC_LD];
+      int* dc = &E.col[pass % BC_STAGES][jr * BC_LD];
+      for (int k = threadIdx.x % T; k < w; k += T) {
+        bc_copy8(dv + k, val + at + 32ll * k);
+        bc_copy4(dc + k, ix + at + 32ll * k);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  // The first pass of a phase over `val` (called before the barrier that opens
+  // the phase: the matrix does not change).
+  __device__ __forceinline__ void begin(const double* val) const {
+    __syncwarp();
+    prefetch(val, 0);
+  }
+  // The entries of `pass` are there; those of the next one are on their way
+  // (into the stage that the pass before used).
+  __device__ __forceinline__ void take(const double* val, int pass) const {
+    __syncwarp();
+    prefetch(val, pass + 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
+  }
+  // acc[e] = sum_k val[row, k] xf(col)[e] for this thread's row of `pass`
+  template <typename F>
+  __device__ __forceinline__ void sum(const double* val, int pass, int row, F xf, double (&acc)[V]) const {
+    const int jr = threadIdx.x / T, sl = (row >> 5) - sl0;
+    const int o = E.off[sl], w = (E.off[sl + 1] - o) >> 5;
+    const double* sv = &E.val[pass % BC_STAGES][jr * BC_LD];
+    const int* sc = &E.col[pass % BC_STAGES][jr * BC_LD];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = 0.0;
+    const int wn = min(w, BC_W);
+#pragma unroll
+    for (int k0 = 0; k0 < BC_W; k0 += 4) {
+      double xv[4][V];
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (k0 + t < wn) xf(sc[k0 + t], xv[t]);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (k0 + t < wn) {
+          const double av = sv[k0 + t];
+#pragma unroll
+          for (int e = 0; e < V; ++e) acc[e] += av * xv[t][e];
+        }
+    }
+    for (int k = BC_W; k < w; ++k) {
+      const long long at = ob + o + (row & 31) + 32ll * k;
+      const double av = __ldg(val + at);
+      double xv[V];
+      xf(__ldg(ix + at), xv);
+#pragma unroll
+      for (int e = 0; e < V; ++e) acc[e] += av * xv[e];
+    }
+  }
+};
+
+// Sums of ND x V values per thread over the rows of a cluster's system; on
+// return red[d * R + q][0] holds right-hand side q's total d for the threads of
+// warp 0.  Everything stored before it is visible to the cluster after it.
+template <int ND, int R>
+__device__ __forceinline__ void bc_sum(double (&v)[ND][vals_per_thread<R>()], double (*red)[BC_THREADS / 32 + 1],
+                                       double (*part)[BC_MAXC], unsigned rank, unsigned C) {
+  constexpr int V = vals_per_thread<R>(), T = R / V, WARPS = BC_THREADS / 32;
+  static_assert(2 * R <= WARPS, "a warp to a sum");
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+#pragma unroll
+  for (int d = 0; d < ND; ++d)
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      double t = v[d][e];
+#pragma unroll
+      for (int o = 16; o >= T; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane < T) red[d * R + lane * V + e][wid] = t;
+    }
+  __syncthreads();
+  if (wid < ND * R) {
+    double t = lane < WARPS ? red[wid][lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane < (int)C)
+      asm volatile("st.shared::cluster.f64 [%0], %1;" : : "r"(bc_remote(&part[wid][rank], (unsigned)lane)), "d"(t)
+                   : "memory");
+  }
+  bc_barrier();
+  if (wid == 0) {
+    if (lane < ND * R) {
+      double t = 0.0;
+      for (unsigned c = 0; c < C; ++c) t += part[lane][c];
+      red[lane][0] = t;  // (the warps' parts were read before the barrier)
+    }
+    __syncwarp();
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(BC_THREADS, 1) k_batch_cluster(BCArgs a) {
+  constexpr int V = vals_per_thread<R>(), T = R / V;
+  constexpr int ROWS = BCEntries<R>::ROWS, THREADS = BC_THREADS;
+  extern __shared__ __align__(16) unsigned char bc_raw[];
+  BCEntries<R>& E = *reinterpret_cast<BCEntries<R>*>(bc_raw);
+  double* bc_sm = reinterpret_cast<double*>(bc_raw + bc_entry_bytes<R>());
+  __shared__ double red[2 * R][BC_THREADS / 32 + 1];
+  __shared__ double part[2][2 * R][BC_MAXC];
+  __shared__ double rho[R], alpha[R], omega[R], beta[R], res[R], thr[R];
+  __shared__ int active[R], stat[R], conv[R];
+  __shared__ int next;
+  const int tid = threadIdx.x;
+  const unsigned rank = bc_rank(), C = bc_size();
+  const int q0 = (tid % T) * V;
+  unsigned par = 0;
+  bc_barrier();  // every CTA of the cluster has started
+
+  // total d of right-hand side tid (threads below R; ND * R <= 32: one warp)
+  auto total = [&](int d) { return red[d * R + tid][0]; };
+
+  for (;;) {
+    if (rank == 0 && tid == 0) {
+      int s = -1;
+      if (atomicAdd(a.head, 1) < a.count)
+        s = (bc_id() & 1) ? a.order[a.count - 1 - atomicAdd(a.head + 2, 1)] : a.order[atomicAdd(a.head + 1, 1)];
+      for (unsigned c = 0; c < C; ++c)
+        asm volatile("st.shared::cluster.s32 [%0], %1;" : : "r"(bc_remote(&next, c)), "r"(s) : "memory");
+    }
+    bc_barrier();
+    const int sys = next;
+    if (sys < 0) break;
+    const int s0 = a.sys_off[sys], s1 = a.sys_off[sys + 1];
+    const int rpc = ((s1 - s0 + (int)C - 1) / (int)C + 7) & ~7;  // rows of a CTA
+    const int c0 = min(s0 + rpc * (int)rank, s1), rows = min(rpc, s1 - c0);
+    const size_t g0 = (size_t)c0 * R;
+    // own-row vectors: shared memory while they fit (the same choice in every CTA)
+    const int need = rpc * R;
+    double* rs = need <= a.cap ? bc_sm : a.rs + g0;
+    double* az = 2 * need <= a.cap ? bc_sm + need : a.az + g0;
+    double* xs = 3 * need <= a.cap ? bc_sm + 2 * need : a.x + g0;
+    const bool x_in = 3 * need <= a.cap;
+
+    // the CTA's slice offsets
+    const int sl0 = c0 >> 5, nsl = rows > 0 ? ((c0 + rows - 1) >> 5) - sl0 + 1 : 0;
+    const long long ob = __ldg(a.off + sl0);
+    for (int t = tid; t <= nsl; t += THREADS) E.off[t] = (int)(__ldg(a.off + sl0 + t) - ob);
+    __syncthreads();
+    const int npass = (rpc + ROWS - 1) / ROWS;
+    const int jr = tid / T;        // this thread's row of a pass
+    const BCRows<R> rw{E, a.off, a.ix, c0, rows, sl0, ob};
+    rw.begin(a.aval);
+
+    // r = b - A x, r* = r, q = 0
+    {
+      double v[2][V] = {};
+      for (int pass = 0; pass < npass; ++pass) {
+        rw.take(a.aval, pass);
+        const int j = pass * ROWS + jr;
+        if (j >= rows) continue;
+        const int row = c0 + j, li = j * R + q0;
+        const size_t i = g0 + li;
+        double ax[V], bb[V], rr[V], zero[V] = {};
+        rw.sum(a.aval, pass, row, [&](int c, double (&o)[V]) { ldp<V>(a.x + (size_t)c * R + q0, o); }, ax);
+        ldv<V>(a.b + i, bb);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          rr[e] = bb[e] + (-1.0) * ax[e];
+          v[0][e] += rr[e] * rr[e];
+          v[1][e] += bb[e] * bb[e];
+        }
+        stv<V>(a.r + i, rr);
+        stv<V>(rs + li, rr);
+        stv<V>(a.q + i, zero);
+        stv<V>(a.ay + i, zero);
+        if (x_in) {
+          double xv[V];
+          ldp<V>(a.x + i, xv);
+          stv<V>(xs + li, xv);
+        }
+      }
+      rw.begin(a.mval);
+      par ^= 1u;
+      bc_sum<2, R>(v, red, part[par], rank, C);
+      if (tid < R) {
+        rho[tid] = total(0);
+        res[tid] = sqrt(total(0));
+        const double bn = sqrt(total(1));
+        thr[tid] = (a.tol_mode == DCU_TOL_REL) ? a.tol * bn : a.tol;
+        alpha[tid] = 0.0;
+        omega[tid] = 1.0;
+        beta[tid] = 0.0;
+        const bool run = res[tid] != 0.0 && a.maxiter > 1;
+        active[tid] = run ? 1 : 0;
+        conv[tid] = 1;
+        stat[tid] = run ? -1 : (res[tid] == 0.0 ? DCU_SOLVE_CONVERGED : DCU_SOLVE_MAXITER);
+      }
+    }
+    int it = 1;
+    int live = __syncthreads_count(tid < R && active[tid < R ? tid : 0]);
+    // a pair that stopped keeps alpha = omega = beta = 0: its x no longer changes
+    auto freeze = [&](int status) {
+      active[tid] = 0;
+      stat[tid] = status;
+      alpha[tid] = omega[tid] = beta[tid] = 0.0;
+    };
+    while (live > 0 && it < a.maxiter) {
+      double be[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) be[e] = beta[q0 + e];
+      // y = M p
+      for (int pass = 0; pass < npass; ++pass) {
+        rw.take(a.mval, pass);
+        const int j = pass * ROWS + jr;
+        if (j >= rows) continue;
+        const int row = c0 + j;
+        double yv[V];
+        rw.sum(a.mval, pass, row, [&](int c, double (&o)[V]) {
+          double rr[V], qq[V];
+          ldp<V>(a.r + (size_t)c * R + q0, rr);
+          ldp<V>(a.q + (size_t)c * R + q0, qq);
+#pragma unroll
+          for (int e = 0; e < V; ++e) o[e] = rr[e] + be[e] * qq[e];
+        }, yv);
+        stv<V>(a.y + g0 + j * R + q0, yv);
+      }
+      rw.begin(a.aval);
+      bc_barrier();
+      // Ay, alpha
+      {
+        double v[1][V] = {};
+        for (int pass = 0; pass < npass; ++pass) {
+          rw.take(a.aval, pass);
+          const int j = pass * ROWS + jr;
+          if (j >= rows) continue;
+          const int row = c0 + j, li = j * R + q0;
+          double t[V], s[V];
+          ldp<V>(rs + li, s);
+          rw.sum(a.aval, pass, row, [&](int c, double (&o)[V]) { ldp<V>(a.y + (size_t)c * R + q0, o); }, t);
+          stv<V>(a.ay + g0 + li, t);
+#pragma unroll
+          for (int e = 0; e < V; ++e) v[0][e] += s[e] * t[e];
+        }
+        rw.begin(a.mval);
+        par ^= 1u;
+        bc_sum<1, R>(v, red, part[par], rank, C);
+        if (tid < R && active[tid]) {
+          const double d = total(0), al = rho[tid] / d;
+          alpha[tid] = al;
+          if (d == 0.0 || !isfinite(al)) freeze(DCU_SOLVE_BREAKDOWN);
+        }
+        __syncthreads();
+      }
+      double na[V];
+#pragma unroll
+      for (int e = 0; e < V; ++e) na[e] = -1.0 * alpha[q0 + e];
+      // z = M s
+      for (int pass = 0; pass < npass; ++pass) {
+        rw.take(a.mval, pass);
+        const int j = pass * ROWS + jr;
+        if (j >= rows) continue;
+        const int row = c0 + j;
+        double zv[V];
+        rw.sum(a.mval, pass, row, [&](int c, double (&o)[V]) {
+          double rr[V], yy[V];
+          ldp<V>(a.r + (size_t)c * R + q0, rr);
+          ldp<V>(a.ay + (size_t)c * R + q0, yy);
+#pragma unroll
+          for (int e = 0; e < V; ++e) o[e] = rr[e] + na[e] * yy[e];
+        }, zv);
+        stv<V>(a.z + g0 + j * R + q0, zv);
+      }
+      rw.begin(a.aval);
+      bc_barrier();
+      // Az, omega
+      {
+        double v[2][V] = {};
+        for (int pass = 0; pass < npass; ++pass) {
+          rw.take(a.aval, pass);
+          const int j = pass * ROWS + jr;
+          if (j >= rows) continue;
+          const int row = c0 + j, li = j * R + q0;
+          double t[V], rr[V], yy[V];
+          ldp<V>(a.r + g0 + li, rr);
+          ldp<V>(a.ay + g0 + li, yy);
+          rw.sum(a.aval, pass, row, [&](int c, double (&o)[V]) { ldp<V>(a.z + (size_t)c * R + q0, o); }, t);
+          stv<V>(az + li, t);
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            v[0][e] += t[e] * (rr[e] + na[e] * yy[e]);
+            v[1][e] += t[e] * t[e];
+          }
+        }
+        rw.begin(a.mval);
+        par ^= 1u;
+        bc_sum<2, R>(v, red, part[par], rank, C);
+        if (tid < R && active[tid]) {
+          // Az = 0 (s = 0 when the half step solved the pair): omega = 0
+          const double om = (total(1) == 0.0) ? 0.0 : total(0) / total(1);
+          omega[tid] = om;
+          if (!isfinite(om)) freeze(DCU_SOLVE_BREAKDOWN);
+        }
+        __syncthreads();
+      }
+      // x, r, q; rho, beta, ||r||
+      {
+        double al[V], om[V], be2[V];
+        bool act[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          al[e] = alpha[q0 + e];
+          om[e] = omega[q0 + e];
+          be2[e] = beta[q0 + e];
+          act[e] = active[q0 + e] != 0;
+        }
+        double v[2][V] = {};
+        for (int j = tid / T; j < rows; j += THREADS / T) {
+          const int li = j * R + q0;
+          const size_t i = g0 + li;
+          double xv[V], yv[V], zv[V], rr[V], qq[V], yy[V], tt[V], s[V];
+          ldp<V>(xs + li, xv);
+          ldp<V>(a.y + i, yv);
+          ldp<V>(a.z + i, zv);
+          ldp<V>(a.r + i, rr);
+          ldp<V>(a.q + i, qq);
+          ldp<V>(a.ay + i, yy);
+          ldp<V>(az + li, tt);
+          ldp<V>(rs + li, s);
+#pragma unroll
+          for (int e = 0; e < V; ++e) {
+            if (act[e]) {
+              const double t = xv[e] + al[e] * yv[e];
+              xv[e] = t + om[e] * zv[e];
+            }
+            const double p = rr[e] + be2[e] * qq[e];
+            const double sv = rr[e] + (-1.0 * al[e]) * yy[e];
+            const double rn = sv + (-1.0 * om[e]) * tt[e];
+            qq[e] = p - om[e] * yy[e];
+            rr[e] = rn;
+            v[0][e] += s[e] * rn;
+            v[1][e] += rn * rn;
+          }
+          stv<V>(xs + li, xv);
+          stv<V>(a.r + i, rr);
+          stv<V>(a.q + i, qq);
+        }
+        par ^= 1u;
+        bc_sum<2, R>(v, red, part[par], rank, C);
+        if (tid < R && active[tid]) {
+          const double rho_new = total(0);
+          const double bt = (rho_new / rho[tid]) * (alpha[tid] / omega[tid]);
+          rho[tid] = rho_new;
+          beta[tid] = bt;
+          res[tid] = sqrt(total(1));
+          conv[tid] = it;
+          // the stop test first, as in the reference (it never examines beta)
+          if (!isfinite(res[tid])) freeze(DCU_SOLVE_BREAKDOWN);
+          else if (res[tid] < thr[tid]) freeze(DCU_SOLVE_CONVERGED);
+          else if (!isfinite(bt) || rho_new == 0.0) freeze(DCU_SOLVE_BREAKDOWN);
+          else if (it + 1 >= a.maxiter) conv[tid] = it + 1;
+        }
+        live = __syncthreads_count(tid < R && active[tid < R ? tid : 0]);
+        ++it;
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (x_in)
+      for (int j = tid / T; j < rows; j += THREADS / T) {
+        double xv[V];
+        ldp<V>(xs + j * R + q0, xv);
+        stv<V>(a.x + g0 + j * R + q0, xv);
+      }
+    if (rank == 0 && tid < R) {
+      a.iters[(size_t)sys * R + tid] = conv[tid];
+      a.status[(size_t)sys * R + tid] = stat[tid] < 0 ? DCU_SOLVE_MAXITER : stat[tid];
+    }
+    __syncthreads();
+  }
+  bc_barrier();  // no CTA leaves while another may still write into its shared memory
+}
+
 __global__ void kb_check_blocks(const int* __restrict__ ptr, const int* __restrict__ idx, const int* __restrict__ sys_off,
                                 int nsys, int n, int* __restrict__ bad) {
   // every column's rows lie in its own diagonal block
@@ -575,6 +1068,145 @@ __global__ void kb_check_blocks(const int* __restrict__ ptr, const int* __restri
   }
 }
 
+// Whether a batch goes to the clusters.  In units of one row x right-hand side
+// of a 16-CTA cluster's iteration (about 0.5 ns; seven such clusters run at
+// once): a cluster's iteration costs its rows and a fixed 20000 (five
+// barriers), the tile kernels' the whole batch's rows at a rate that grows with
+// the right-hand sides (they are bound by HBM, the clusters by L1) and a fixed
+// 48000 (six launches).  Measured on one B200, tile kernels -> clusters: 128 systems
+// of 300-4000 rows x 8 6.9 -> 4.3 ms, 256 of 300-50000 x 4 53.9 -> 44.1, x 2 37.1 ->
+// 24.5, x 1 32.6 -> 19.4, 16 small ones 2.6 -> 1.1; 512 of 1000-50000 x 8 equal, 8 of
+// 300-50000 x 4 9.0 -> 9.7 (too few large systems to fill the clusters).
+template <int R>
+bool cluster_batch(const std::vector<int>& so, int nsys) {
+  double sum = 0.0, most = 0.0;
+  int rows = 0;
+  for (int s = 0; s < nsys; ++s) {
+    const int n = so[s + 1] - so[s];
+    rows = std::max(rows, n);
+    sum += (double)n * R;
+    most = std::max(most, 20000.0 + (R <= 2 ? 0.6 : 1.0) * n * R);
+  }
+  if (rows > BC_MAXC * (32 * (BC_SLICES - 2) - 8)) return false;  // slices of a CTA
+  return std::max(sum / 7.0, most) < 48000.0 + sum * (R == 8 ? 0.14 : R == 4 ? 0.17 : 0.3);
+}
+
+// The systems of a batch through k_batch_cluster: classes by size, the larger
+// the system the more CTAs share it.  *ran stays false when the device cannot
+// hold the clusters.
+template <int R>
+int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector<int>& so, const SellPlan& plan,
+                       const double* aval, const double* mval, const double* B, double* X, const dcu_options* opt,
+                       int* iters_h, int* status_h, dcu_solve_info* info, bool* ran) {
+  const int n = plan.n;
+  auto kernel = k_batch_cluster<R>;
+  // shared memory: the entries, then the rows' own vectors (more of it made no
+  // difference: 60, 120 and 210 KB within 1%)
+  const size_t smem = std::max<size_t>(64 * 1024, bc_entry_bytes<R>());
+  if (smem + 16 * 1024 > c->smem_optin) return DCU_OK;
+  DCU_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  DCU_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  std::vector<int> order(nsys);
+  for (int s = 0; s < nsys; ++s) order[s] = s;
+  std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return so[p + 1] - so[p] > so[q + 1] - so[q]; });
+  // CTAs per system: two passes of rows each, up to 16
+  const int unit = BCEntries<R>::ROWS;
+  auto ctas = [&](int rows) {
+    int k = 1;
+    while (k < BC_MAXC && rows > 2 * unit * k) k <<= 1;
+    return k;
+  };
+  struct Class {
+    int cta, first, count, grid;
+  };
+  std::vector<Class> cls;
+  for (int i = 0; i < nsys; ++i) {
+    const int k = ctas(so[order[i] + 1] - so[order[i]]);
+    if (cls.empty() || cls.back().cta != k) cls.push_back({k, i, 0, 0});
+    ++cls.back().count;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(BC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  for (auto& k : cls) {
+    int fit = 0;
+    at[0].val.clusterDim.x = k.cta;
+    cfg.gridDim = dim3(k.cta);
+    if (cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      return DCU_OK;
+    }
+    k.grid = std::min(fit, k.count) * k.cta;
+  }
+  auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
+  const size_t vec = al(sizeof(double) * (size_t)n * R), pairs = (size_t)nsys * R;
+  const size_t heads = al(sizeof(int) * 3 * cls.size());
+  DCU_TRY(ensure(c, B_VEC, 7 * vec + heads + al(sizeof(int) * nsys) + 2 * al(sizeof(int) * pairs)));
+  char* p = bp<char>(c, B_VEC);
+  BCArgs a{};
+  a.sys_off = sys_off_d;
+  a.off = plan.off;
+  a.kd = plan.kd;
+  a.su = plan.su;
+  a.ix = plan.idx;
+  a.aval = aval;
+  a.mval = mval;
+  a.b = B;
+  a.x = X;
+  double** vecs[7] = {&a.r, &a.q, &a.y, &a.ay, &a.z, &a.rs, &a.az};
+  for (int i = 0; i < 7; ++i) *vecs[i] = reinterpret_cast<double*>(p + i * vec);
+  int* head = reinterpret_cast<int*>(p + 7 * vec);
+  int* ord = reinterpret_cast<int*>(p + 7 * vec + heads);
+  a.iters = reinterpret_cast<int*>(p + 7 * vec + heads + al(sizeof(int) * nsys));
+  a.status = reinterpret_cast<int*>(p + 7 * vec + heads + al(sizeof(int) * nsys) + al(sizeof(int) * pairs));
+  a.tol = opt->tol;
+  a.tol_mode = opt->tol_mode;
+  a.maxiter = opt->maxiter > 0 ? opt->maxiter : n;
+  a.cap = (int)((smem - bc_entry_bytes<R>()) / sizeof(double));
+  DCU_CUDA(c, cudaMemsetAsync(head, 0, heads, c->stream));
+  DCU_CUDA(c, cudaMemcpyAsync(ord, order.data(), sizeof(int) * nsys, cudaMemcpyHostToDevice, c->stream));
+  DCU_CUDA(c, cudaEventRecord(c->ev[0], c->stream));
+  // every second class on the auxiliary stream: its clusters start as the
+  // larger systems' last ones leave the SMs
+  DCU_CUDA(c, cudaEventRecord(c->ev[6], c->stream));
+  DCU_CUDA(c, cudaStreamWaitEvent(c->aux_stream, c->ev[6], 0));
+  for (size_t k = 0; k < cls.size(); ++k) {
+    a.count = cls[k].count;
+    a.order = ord + cls[k].first;
+    a.head = head + 3 * k;
+    at[0].val.clusterDim.x = cls[k].cta;
+    cfg.gridDim = dim3(cls[k].grid);
+    cfg.stream = (k & 1) ? c->aux_stream : c->stream;
+    DCU_CUDA(c, cudaLaunchKernelEx(&cfg, kernel, a));
+    c->launches++;
+  }
+  DCU_CUDA(c, cudaEventRecord(c->ev[7], c->aux_stream));
+  DCU_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev[7], 0));
+  DCU_CUDA(c, cudaEventRecord(c->ev[1], c->stream));
+  DCU_CUDA(c, cudaMemcpyAsync(iters_h, a.iters, sizeof(int) * pairs, cudaMemcpyDeviceToHost, c->stream));
+  DCU_CUDA(c, cudaMemcpyAsync(status_h, a.status, sizeof(int) * pairs, cudaMemcpyDeviceToHost, c->stream));
+  DCU_CUDA(c, cudaStreamSynchronize(c->stream));
+  *ran = true;
+  if (info) {
+    info->iters = 1;
+    info->status = DCU_SOLVE_CONVERGED;
+    for (size_t i = 0; i < pairs; ++i) {
+      info->iters = std::max(info->iters, iters_h[i]);
+      info->status = std::max(info->status, status_h[i]);
+    }
+    info->replacements = 0;
+    info->res = info->true_res = info->bnorm = 0.0;
+    info->a_fp32 = 0;
+    cudaEventElapsedTime(&info->ms, c->ev[0], c->ev[1]);
+  }
+  return DCU_OK;
+}
+
 template <int R>
 int run_batch(Ctx* c, int nsys, const int* sys_off_d, const SellPlan& plan, const double* aval, const double* mval,
               const double* B, double* X, const dcu_options* opt, int* iters_h, int* status_h,
@@ -584,6 +1216,11 @@ int run_batch(Ctx* c, int nsys, const int* sys_off_d, const SellPlan& plan, cons
   std::vector<int> so(nsys + 1);
   DCU_CUDA(c, cudaMemcpyAsync(so.data(), sys_off_d, sizeof(int) * (nsys + 1), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (cluster_batch<R>(so, nsys)) {
+    bool ran = false;
+    DCU_TRY(run_batch_clusters<R>(c, nsys, sys_off_d, so, plan, aval, mval, B, X, opt, iters_h, status_h, info, &ran));
+    if (ran) return DCU_OK;
+  }
   std::vector<int> tsys, trow, toff(nsys + 1, 0);
   for (int s = 0; s < nsys; ++s) {
     toff[s] = (int)tsys.size();
