@@ -207,8 +207,8 @@ struct SellPlan {
   const int* rptr = nullptr;  // CSR row pointers of the laid-out operator (row lengths)
   const int* wide = nullptr;  // the slices flagged wide (device)
   int nwide = 0;
-  // one-launch solver (persist.cu): most slots and most long rows any of its
-  // blocks holds; 0 slots when it does not take an operator of this size
+  // one-launch solver (persist.cu): most slots and most segments of long rows
+  // any of its blocks holds; 0 slots when it does not take an operator of this size
   int max_block_slots = 0, max_block_long = 0;
 };
 
@@ -219,6 +219,7 @@ struct PersistShape {
   int spb = 0, blocks = 0;
 };
 constexpr int kPersistLong = 16;     // a longer row of a wide slice is summed by a warp
+constexpr int kPersistSeg = 128;     // entries of such a row that one warp takes at a time
 constexpr int kPersistBlocks = 160;  // most blocks (a multiple of 32)
 PersistShape persist_shape(const Ctx* c, int n);
 

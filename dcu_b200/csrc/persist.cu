@@ -116,10 +116,10 @@ struct PSmem {
   double* q;
   double* ay;
   double* yz;
-  double* lval;      // [cap_long] sums of the long rows
+  double* lval;      // [cap_long] sums of the long rows' segments
   MT* m;             // [cap_slots] M's entries
   unsigned* e;       // [cap_slots] column (grid) or shared::cluster address of r[column]
-  int* lstart;       // [cap_long]
+  int* lstart;       // [cap_long] a segment's entries
   int* llen;         // [cap_long]
 };
 
@@ -157,7 +157,8 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   constexpr int PW = PT / 32;
   extern __shared__ __align__(16) unsigned char p_raw[];
   __shared__ int sbase[kPSlices + 1];
-  __shared__ int slong[2];                 // long rows, their entries
+  __shared__ int slong[2];                 // segments of long rows, their entries
+  __shared__ int ticket;                   // next segment to sum
   __shared__ double red[2][PW];
   __shared__ double sums[2];               // grid form: the totals
   __shared__ double part[2][2][16];        // cluster form: [parity][sum][rank]
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   // the end): its rows longer than kPLong go to the long list, a warp to a
   // row, and the others set its width.
   if (tid < 2) slong[tid] = 0;
+  if (tid == 0) ticket = 0;
   __syncthreads();
   auto slice_len = [&](int s, int w, bool& split) {  // this lane's row length; whether long rows leave the slice
     const int r = s * 32 + lane;
@@ -228,7 +230,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     S.m[dst] = mv;
     S.e[dst] = CL ? p_mapa(base_r + 8u * (unsigned)(c % rows_pb), (unsigned)(c / rows_pb)) : (unsigned)c;
   };
-  int li[RPT];  // index of the row's sum in lval, or -1
+  int li[RPT];  // a long row's first segment in lval and their number << 16, or -1
 #pragma unroll
   for (int j = 0; j < RPT; ++j) {
     li[j] = -1;
@@ -264,21 +266,22 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       const int jl = __ffs(longs) - 1;
       longs &= longs - 1;
       const int L = __shfl_sync(0xffffffffu, len, jl);
+      const int nseg = (L + kPersistSeg - 1) / kPersistSeg;
       int l = 0, st = 0;
       if (lane == 0) {
-        l = atomicAdd(&slong[0], 1);
+        l = atomicAdd(&slong[0], nseg);
         st = lbase + atomicAdd(&slong[1], L);
       }
       l = __shfl_sync(0xffffffffu, l, 0);
       st = __shfl_sync(0xffffffffu, st, 0);
-      if (l >= a.cap_long) {
+      if (l + nseg > a.cap_long) {
         err = P_ERR_CAPACITY;
         continue;
       }
-      if (lane == jl) li[j] = l;
-      if (lane == 0) {
-        S.lstart[l] = st;
-        S.llen[l] = L;
+      if (lane == jl) li[j] = l | (nseg << 16);
+      for (int g = lane; g < nseg; g += 32) {
+        S.lstart[l + g] = st + g * kPersistSeg;
+        S.llen[l + g] = min(kPersistSeg, L - g * kPersistSeg);
       }
       for (int k = lane; k < L; k += 32) {
         int cv;
@@ -313,7 +316,6 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   auto x_s = [&](unsigned e) { return g_r(e) + nalpha * g_ay(e); };
   // this thread's row j: sum over its entries, eight gathers in flight
   auto row_dot = [&](int j, auto vals, auto xf) {
-    if (li[j] >= 0) return S.lval[li[j]];
     const int t = wid + j * PW;
     const int o = sbase[t], w = sbase[t + 1] - o;
     const int at = o * 32 + lane;
@@ -328,25 +330,41 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     }
     return acc;
   };
-  // the long rows first, a warp per row
-  auto long_rows = [&](auto vals, auto xf) {
+  const int row0 = s0 * 32;
+  auto row_of = [&](int j) { return row0 + tid + j * PT; };
+  auto mine = [&](int j) { return tid + j * PT < ns * 32 && row_of(j) < a.n; };
+  // The block's rows: each thread its own, then the long rows' segments of
+  // kPersistSeg entries, a warp to a segment, by ticket (warps without rows of
+  // their own start there at once); a long row adds its segments in order.
+  auto rows_dot = [&](auto vals, auto xf, double (&out)[RPT]) {
+#pragma unroll
+    for (int j = 0; j < RPT; ++j) out[j] = mine(j) && li[j] < 0 ? row_dot(j, vals, xf) : 0.0;
     if (nlong == 0) return;
-    for (int l = wid; l < nlong; l += PW) {
+    __syncwarp();
+    for (;;) {
+      int l = 0;
+      if (lane == 0) l = atomicAdd(&ticket, 1);
+      l = __shfl_sync(0xffffffffu, l, 0);
+      if (l >= nlong) break;
       const int st = S.lstart[l], L = S.llen[l];
-      double acc = 0.0;
-      for (int k0 = lane; k0 < L; k0 += 128) {
-        double xv[4];
+      double xv[kPersistSeg / 32], acc = 0.0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) xv[u] = (k0 + 32 * u < L) ? xf(S.e[st + k0 + 32 * u]) : 0.0;
+      for (int u = 0; u < kPersistSeg / 32; ++u) xv[u] = (lane + 32 * u < L) ? xf(S.e[st + lane + 32 * u]) : 0.0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (k0 + 32 * u < L) acc += (double)vals[st + k0 + 32 * u] * xv[u];
-      }
+      for (int u = 0; u < kPersistSeg / 32; ++u)
+        if (lane + 32 * u < L) acc += (double)vals[st + lane + 32 * u] * xv[u];
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
       if (lane == 0) S.lval[l] = acc;
     }
     __syncthreads();
+    if (tid == 0) ticket = 0;
+#pragma unroll
+    for (int j = 0; j < RPT; ++j)
+      if (li[j] >= 0) {
+        const int l = li[j] & 0xffff, m = li[j] >> 16;
+        for (int g = 0; g < m; ++g) out[j] += S.lval[l + g];
+      }
   };
 
   // ---- barrier with up to two sums -----------------------------------------
@@ -385,18 +403,12 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       }
       p_cluster_barrier();
       if (nd > 0) {
+        // lanes 0-15 the first sum's parts, 16-31 the second's
+        double t = (lane & 15) < a.blocks ? part[par][lane >> 4][lane & 15] : 0.0;
 #pragma unroll
-        for (int d = 0; d < 2; ++d) {
-          if (d >= nd) break;
-          double s[16];
-#pragma unroll
-          for (int w = 0; w < 16; ++w) s[w] = w < a.blocks ? part[par][d][w] : 0.0;
-#pragma unroll
-          for (int h = 8; h > 0; h >>= 1)
-#pragma unroll
-            for (int w = 0; w < h; ++w) s[w] += s[w + h];
-          tot[d] = s[0];
-        }
+        for (int h = 8; h > 0; h >>= 1) t += __shfl_xor_sync(0xffffffffu, t, h);
+        tot[0] = __shfl_sync(0xffffffffu, t, 0);
+        tot[1] = __shfl_sync(0xffffffffu, t, 16);
       }
       return true;
     } else {
@@ -483,9 +495,6 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   };
 
   // ---- the solve ------------------------------------------------------------
-  const int row0 = s0 * 32;
-  auto row_of = [&](int j) { return row0 + tid + j * PT; };
-  auto mine = [&](int j) { return tid + j * PT < ns * 32 && row_of(j) < a.n; };
   auto put_rq = [&](int j, double rv, double qv) {
     if (CL) {
       S.r[tid + j * PT] = rv;
@@ -518,15 +527,14 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     for (int j = 0; j < RPT; ++j)
       if (mine(j)) put_yz(j, x[j]);
     if (!sync(0, 0.0, 0.0)) return false;
-    long_rows(S.a, g_yz);
+    rows_dot(S.a, g_yz, v);
     double d0 = 0.0, d1 = 0.0;
     bb = 0.0;
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
-      v[j] = 0.0;
       if (!mine(j)) continue;
       const double br = a.b[row_of(j)];
-      v[j] = br - row_dot(j, S.a, g_yz);
+      v[j] = br - v[j];
       if (first) rs[j] = v[j];
       d0 += rs[j] * v[j];
       d1 += v[j] * v[j];
@@ -555,11 +563,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   }
   while (ok && status < 0) {
     // y = M p
-    long_rows(S.m, x_p);
+    rows_dot(S.m, x_p, y);
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
       if (!mine(j)) continue;
-      y[j] = row_dot(j, S.m, x_p);
       const double qv = p[j] - omega * ay[j];
       p[j] = r[j] + beta * qv;
       put_yz(j, y[j]);
@@ -567,11 +574,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     if (!(ok = sync(0, 0.0, 0.0))) break;
     // Ay, alpha
     double d0 = 0.0, d1 = 0.0;
-    long_rows(S.a, g_yz);
+    rows_dot(S.a, g_yz, ay);
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
       if (!mine(j)) continue;
-      ay[j] = row_dot(j, S.a, g_yz);
       put_ay(j, ay[j]);
       d0 += rs[j] * ay[j];
     }
@@ -583,11 +589,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     }
     // s = r - alpha Ay (kept in r), z = M s
     nalpha = -1.0 * alpha;
-    long_rows(S.m, x_s);
+    rows_dot(S.m, x_s, z);
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
       if (!mine(j)) continue;
-      z[j] = row_dot(j, S.m, x_s);
       r[j] = r[j] + nalpha * ay[j];
       put_yz(j, z[j]);
     }
@@ -595,12 +600,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     // Az, omega
     d0 = d1 = 0.0;
     double az[RPT];
-    long_rows(S.a, g_yz);
+    rows_dot(S.a, g_yz, az);
 #pragma unroll
     for (int j = 0; j < RPT; ++j) {
-      az[j] = 0.0;
       if (!mine(j)) continue;
-      az[j] = row_dot(j, S.a, g_yz);
       d0 += az[j] * r[j];
       d1 += az[j] * az[j];
     }

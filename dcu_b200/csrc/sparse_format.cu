@@ -362,12 +362,12 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       kd8h[(long long)s * kNarrow + lane] = (int16_t)d;  // read only when every |d| < 32768
     }
     // the slice's share of a block of the one-launch solver (persist.cu, which
-    // makes the same split): slots kept, entries and number of the long rows
+    // makes the same split): slots kept, entries and segments of the long rows
     if (spb > 0) {
       const bool split = w > kPersistLong && few_long;
       const int ws = __reduce_max_sync(0xffffffffu, !split ? w : (len <= kPersistLong ? len : 0));
       const int le = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? len : 0);
-      const int nl = __popc(__ballot_sync(0xffffffffu, split && len > kPersistLong));
+      const int nl = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? (len + kPersistSeg - 1) / kPersistSeg : 0);
       if (lane == 0) {
         atomicAdd(&cost[2 * (s / spb)], 32 * ws + le);
         if (nl) atomicAdd(&cost[2 * (s / spb) + 1], nl);
@@ -695,7 +695,8 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_TRY(ensure(c, B_SELL_KD, sizeof(int) * ((size_t)nslices + (size_t)(slots / 32) + 1)));
   int* su = bp<int>(c, B_SELL_KD);
   int* kd = su + nslices;
-  // slots, uniform slots; then per block of the one-launch solver its slots and long rows
+  // slots, uniform slots; then per block of the one-launch solver its slots and
+  // segments of long rows
   const PersistShape ps = persist_shape(c, n);
   unsigned long long hst[2 + kPersistBlocks] = {(unsigned long long)slots};
   const size_t nst = sizeof(unsigned long long) * (2 + (size_t)ps.blocks);
