@@ -313,10 +313,6 @@ template <typename MT, typename IT, typename VT, typename F>
 __device__ __forceinline__ double a_row(const BiArgs<MT, IT, VT>& a, int r, F xf) {
   return sell_row<false, double, IT>(a.off, a.kd, a.kd8, a.kd8h, a.su, a.wide_val, a.aval, nullptr, a.ix, r, xf);
 }
-// The plain FP64 form (FP64 M) never reads A's FP32 copy.
-template <typename MT>
-constexpr bool kA32 = !std::is_same<MT, double>::value;
-
 // A's row from the FP32 copy of its values: the same numbers when every
 // value of A is exact in FP32 (Scal::a32), widened to FP64 before the
 // multiply, so the row's sum is bit-identical to a_row's.
@@ -472,7 +468,7 @@ __global__ void __launch_bounds__(BI_BLOCK) k_bi_init(BiArgs<MT, IT, VT> a, doub
                                                       int verify) {
   double v[3] = {0.0, 0.0, 0.0};
   // with every value of A exact in FP32 its FP64 SELL copy may be absent
-  const bool a32 = kA32<MT> && a.aval32 && *a.a_inexact == 0;
+  const bool a32 = a.aval32 && *a.a_inexact == 0;
   auto xf = [&](int c) { return ldv(a.x + c); };
   const int stride = gridDim.x * BI_BLOCK;
   for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
@@ -538,15 +534,15 @@ __global__ void __launch_bounds__(BI_BLOCK) k_bi_py(BiArgs<MT, IT, VT> a) {
   }
 }
 
-// Split form of K1, used with a narrow (FP32 / BF16) preconditioner: p is
-// formed once per row by a streaming kernel and then read by a one-vector
-// SpMV, instead of at every gathered column (three gathered vectors per
-// entry).  Same arithmetic as the fused kernel.  This is the untuned default:
-// split with a narrow M, fused with an FP64 M (whose SpMV moves 8 bytes of
-// value per entry, so the gathers the split saves weigh less).  The autotuner
-// compares both in whole solves where they compute the same values (FP64
-// vectors); at 128^3 it finds the split faster with an FP64 M too.  K3
-// gathers two vectors and stays fused always.
+// Split form of K1: p is formed once per row by a streaming kernel and then
+// read by a one-vector SpMV, instead of at every gathered column (three
+// gathered vectors per entry).  Same arithmetic as the fused kernel.  The
+// untuned default: split with a narrow (FP32 / BF16) M, and with an FP64 M and
+// FP64 vectors from kSplitNnz entries on, where the gathers cost more than the
+// extra launch (128^3: 169 against 175 us an iteration); fused below.  The
+// autotuner compares both in whole solves where they compute the same values
+// (FP64 vectors).  K3 gathers two vectors and stays fused always.
+constexpr long long kSplitNnz = 1ll << 22;
 template <typename MT>
 constexpr bool split_k1() {
   return !std::is_same<MT, double>::value;
@@ -595,8 +591,9 @@ __global__ void __launch_bounds__(BI_BLOCK, 8) k_bi_y(BiArgs<MT, IT, VT> a) {
 
 // K2: ay = A y; alpha = rho / (r*, ay)
 // 32 registers (8 blocks per SM) with 16-bit columns and a narrow M; with
-// int32 columns or an FP64 M up to 48 without spilling (5 blocks).  (An
-// explicit minimum of one block lets the compiler take 64 for the former.)
+// int32 columns or an FP64 M up to 48 (5 blocks; K4 alike, 56 without the
+// bound).  At 8 blocks the FP64 form gains 0.4% at 128^3 and loses 9% at 75^3.
+// (An explicit minimum of one block lets the compiler take 64 for the former.)
 template <typename MT, typename IT, typename VT>
 __global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || std::is_same<IT, int>::value) ? 5 : 8)
     k_bi_ay(BiArgs<MT, IT, VT> a) {
@@ -612,7 +609,7 @@ __global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || 
     v[0] += rsv * ayv;
   };
   const VT* __restrict__ rs = a.rs;
-  if (kA32<MT> && a.S->a32) {
+  if (a.S->a32) {
     for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
       const double rsv = ldv(rs + r);
       row(r, rsv, a_row32(a, r, yf));
@@ -655,7 +652,8 @@ __global__ void __launch_bounds__(BI_BLOCK) k_bi_sz(BiArgs<MT, IT, VT> a) {
 
 // K4: az = A z; omega = (az, s) / (az, az)
 template <typename MT, typename IT, typename VT>
-__global__ void __launch_bounds__(BI_BLOCK) k_bi_az(BiArgs<MT, IT, VT> a) {
+__global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || std::is_same<IT, int>::value) ? 5 : 8)
+    k_bi_az(BiArgs<MT, IT, VT> a) {
   if (finished(a.S)) return;
   double v[2] = {0.0, 0.0};
   const VT* __restrict__ z = a.z;
@@ -669,7 +667,7 @@ __global__ void __launch_bounds__(BI_BLOCK) k_bi_az(BiArgs<MT, IT, VT> a) {
     v[1] += azv * azv;
   };
   const double* __restrict__ s = a.s;
-  if (kA32<MT> && a.S->a32) {
+  if (a.S->a32) {
     for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
       const double sv = ldv(s + r);
       row(r, sv, a_row32(a, r, zf));
@@ -768,7 +766,7 @@ __global__ void __launch_bounds__(BI_BLOCK, 6) k_bi_xr(BiArgs<MT, IT, VT> a) {
 template <typename MT, typename IT, typename VT>
 __global__ void __launch_bounds__(BI_BLOCK) k_bi_true(BiArgs<MT, IT, VT> a, int replace) {
   double v[2] = {0.0, 0.0};
-  const bool a32 = kA32<MT> && a.S->a32;  // (k_bi_init decided it)
+  const bool a32 = a.S->a32;  // (k_bi_init decided it)
   auto xf = [&](int c) { return ldv(a.x + c); };
   const int stride = gridDim.x * BI_BLOCK;
   for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
@@ -877,7 +875,8 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
   // vectors are FP64 (the fused step's p is exact in VT); with FP32 vectors
   // the fused step multiplies by the unrounded p, so the form keeps its split.
   constexpr bool k1_free = std::is_same<VT, double>::value;
-  const bool split = (k1_free && tu && tu->k1_split >= 0) ? tu->k1_split == 1 : split_k1<MT>();
+  const bool dsplit = split_k1<MT>() || (k1_free && (long long)plan.nnz >= kSplitNnz);
+  const bool split = (k1_free && tu && tu->k1_split >= 0) ? tu->k1_split == 1 : dsplit;
   // vectors: r, ay, s, az (double) + rs, p0, p1, y, z (VT), 256-byte aligned
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t nd = al(sizeof(double) * (size_t)n), nv = al(sizeof(VT) * (size_t)n);
@@ -932,7 +931,7 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
     c->profile_sel = {sel[IK_PY], 0, sel[IK_SZ], 0, 0};
   }
   c->profile_k1_free = k1_free;
-  c->profile_default_split = split_k1<MT>() ? 1 : 0;
+  c->profile_default_split = dsplit ? 1 : 0;
   c->profile_launch = [c, a, grid_of](int kind, int s) -> int {
     const int g = grid_of(kind, s);
     DCU_CUDA(c, cudaMemsetAsync(&a.S->done, 0, sizeof(int), c->stream));

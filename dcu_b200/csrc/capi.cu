@@ -55,15 +55,18 @@ int resolve_range(Ctx* c, int n, const dcu_options* in, dcu_options* out) {
   return DCU_OK;
 }
 
-// A's values (FP64) in SELL order, and for the forms other than plain FP64
-// (which reads FP64 values, as it reads int32 indices), unless
-// dcu_set_exact_a32 turned it off, the FP32 copy with its exactness flag.
+// A's values in SELL order: FP64, and, unless dcu_set_exact_a32 turned it off,
+// the FP32 copy with its exactness flag for the forms other than plain FP64
+// and for the plain form from kA32Slots on (there an iteration is bound by
+// HBM and A's values are a quarter of its bytes: 128^3 FP64 169 -> 150 us;
+// below, the check and the copy cost what they save).
+constexpr long long kA32Slots = 1ll << 22;
 int gather_a(Ctx* c, const dcu::SellPlan& plan, const double* val, int precision, dcu::SellA* a) {
   const size_t slots = (size_t)(plan.slots > 0 ? plan.slots : 1);
   DCU_TRY(dcu::ensure(c, dcu::B_SELL_AVAL, sizeof(double) * slots));
   *a = dcu::SellA{};
   a->v64 = dcu::bp<double>(c, dcu::B_SELL_AVAL);
-  if (!c->exact_a32 || precision == DCU_PREC_FP64)
+  if (!c->exact_a32 || (precision == DCU_PREC_FP64 && plan.slots < kA32Slots))
     return dcu::sell_gather_f64(c, plan, val, dcu::bp<double>(c, dcu::B_SELL_AVAL));
   DCU_TRY(dcu::ensure(c, dcu::B_SELL_AVAL32, sizeof(float) * slots));
   DCU_TRY(dcu::ensure(c, dcu::B_SELL_AFLAG, sizeof(int)));

@@ -337,8 +337,37 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   // kPersistSeg entries, a warp to a segment, by ticket (warps without rows of
   // their own start there at once); a long row adds its segments in order.
   auto rows_dot = [&](auto vals, auto xf, double (&out)[RPT]) {
+    if constexpr (RPT == 2) {
+      // both rows' gathers in flight together (four rows: spills, slower)
+      int at[2], w[2];
+      double acc[2] = {0.0, 0.0};
 #pragma unroll
-    for (int j = 0; j < RPT; ++j) out[j] = mine(j) && li[j] < 0 ? row_dot(j, vals, xf) : 0.0;
+      for (int i = 0; i < 2; ++i) {
+        const int t = wid + i * PW;
+        const bool in = mine(i) && li[i] < 0;
+        const int o = in ? sbase[t] : 0;
+        w[i] = in ? sbase[t + 1] - o : 0;
+        at[i] = o * 32 + lane;
+      }
+      const int wm = max(w[0], w[1]);
+      for (int k0 = 0; k0 < wm; k0 += 8) {
+        double xv[2][8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) xv[i][u] = (k0 + u < w[i]) ? xf(S.e[at[i] + 32 * (k0 + u)]) : 0.0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (k0 + u < w[i]) acc[i] += (double)vals[at[i] + 32 * (k0 + u)] * xv[i][u];
+      }
+      out[0] = acc[0];
+      out[1] = acc[1];
+    } else {
+#pragma unroll
+      for (int j = 0; j < RPT; ++j) out[j] = mine(j) && li[j] < 0 ? row_dot(j, vals, xf) : 0.0;
+    }
     if (nlong == 0) return;
     __syncwarp();
     for (;;) {

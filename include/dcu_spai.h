@@ -125,8 +125,8 @@ typedef struct {
   double true_res;        /* ||b - A x||_2 recomputed in FP64 at exit                  */
   double bnorm;           /* ||b||_2                                                   */
   float ms;               /* device time of the solve (CUDA events)                   */
-  int a_fp32;             /* 1 when the A products read A's FP32 copy (a form other than
-                             DCU_PREC_FP64, every value of A exact in FP32;
+  int a_fp32;             /* 1 when the A products read A's FP32 copy (every value of A exact
+                             in FP32; DCU_PREC_FP64 only for large operators;
                              dcu_set_exact_a32)                                        */
 } dcu_solve_info;
 
@@ -314,16 +314,15 @@ int dcu_sell_plan_stats(dcu_spai_ctx* ctx, long long* slots, long long* uniform_
  * pre-pass.  No counterpart in the reference. */
 int dcu_set_wide_prepass(dcu_spai_ctx* ctx, int enabled);
 
-/* Let this context's later solves in the forms other than DCU_PREC_FP64 read
- * A's values from an FP32 copy when every value of A is exactly an FP32
+/* Let this context's later solves in the forms other than DCU_PREC_FP64, and
+ * in DCU_PREC_FP64 from 2^22 stored slots on, read A's values from an FP32 copy when every value of A is exactly an FP32
  * number (enabled != 0, the default), or always from the FP64 array (0).
  * The check runs on the device while A is laid out for the solver; the
  * products are formed in FP64 from the same numbers either way, so the
  * iterates are bit-identical, and a matrix with one value that FP32 rounds
  * keeps the FP64 reads.  Integer and dyadic stencil coefficients qualify;
- * values read from decimal text usually do not.  The plain FP64 form always
- * reads FP64 values (as it always reads int32 indices).  No counterpart in
- * the reference. */
+ * values read from decimal text usually do not.  No counterpart in the
+ * reference. */
 int dcu_set_exact_a32(dcu_spai_ctx* ctx, int enabled);
 
 /* ---- autotuner (no counterpart in the reference) ----------------------------- */
@@ -334,8 +333,8 @@ int dcu_set_exact_a32(dcu_spai_ctx* ctx, int enabled);
  * k blocks per SM (capped at what fits).  A row's arithmetic does not depend
  * on the grid, and the two first steps compute the same values, so every
  * field except group_max_ni leaves the solution bit-identical:
- *   k1_split   -1: the form's default (split with an FP32 / BF16 M, fused
- *              with an FP64 M); 0: fused (p formed at every gathered column
+ *   k1_split   -1: the form's default (split with an FP32 / BF16 M and, from
+ *              2^22 entries on, with an FP64 M; else fused); 0: fused (p formed at every gathered column
  *              inside y = M p); 1: split (a p pass, then y = M p).  Forms with
  *              FP32 vectors keep their default: their fused step multiplies
  *              by the unrounded p, so the two differ in rounding there.
