@@ -54,6 +54,7 @@ enum BufId {
   B_PLANSTAT,      // slots of the last SELL plan in offset-uniform slices
   B_HUBPOOL,       // slabs of the columns factored by the hub kernels
   B_HUBMETA,       // their descriptors
+  B_HUBT,          // FP64 hub panels: block reflectors' T, block counts
   B_HUBWPRE,       // prefix of their widths (warp -> column map)
   B_SELL_WIDE,     // SELL: count and list of the slices wider than kWideSlice
   B_WIDEVAL,       // solver: row values of those slices, from the wide pre-pass

@@ -1789,6 +1789,232 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_step(HubArgs h, int c, int 
   }
 }
 
+// ---- FP64 hub columns by panels --------------------------------------------
+// k_hub_step re-reads and rewrites every trailing column for every reflector:
+// one launch per step, bound by L2 (circuit-like matrix, 400 steps: 2.4 ms on one B200).
+// Here a panel of up to HUB_PANEL columns is factored by one CTA per hub, with
+// the triangular factor T of its block reflector I - V T V^T, and one launch
+// applies it to all trailing columns: a column crosses L2 once per panel, and
+// two launches replace eight.
+// The forms with FP32 vectors keep the FP32 steps: their iterates follow every
+// rounding of M.
+constexpr int HUB_PANEL = 8;
+constexpr int HUB_PANEL_THREADS = 512;
+constexpr int HUB_PANEL_RP = 4;       // rows per thread of the panel kernel
+constexpr int HUB_TALL = HUB_PANEL_THREADS * HUB_PANEL_RP;  // tallest block taken by panels
+constexpr int HUB_UP_THREADS = 256;
+constexpr int HUB_UP_COLS = 4;        // trailing columns per warp
+constexpr int HUB_UP_BLOCK = HUB_UP_COLS * HUB_UP_THREADS / 32;
+
+// Householder factorisation of columns c0 .. c0 + width - 1 of every active hub
+// (one block per hub), rows c0 on, in registers: a thread holds HUB_PANEL_RP
+// rows of all the panel's columns.  A step takes one block reduction: the
+// column's products with itself, with the columns after it and with the
+// reflectors before it (v = a - alpha e_c, so v^T a_j = a^T a_j - alpha a_j[c]).
+// tq: HUB_PANEL^2 per hub, T by rows.
+__global__ void __launch_bounds__(HUB_PANEL_THREADS) k_hub_panel(HubArgs h, int c0, double* __restrict__ tq) {
+  constexpr int P = HUB_PANEL, W = HUB_PANEL_THREADS / 32;
+  __shared__ double red[P][W + 1], tot[P], prow[P], T[P][P];
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const HubMeta hm = h.meta[blockIdx.x];
+  const int m = hm.m, steps = min(hm.nj, m);
+  cudaGridDependencySynchronize();
+  if (c0 >= steps) return;
+  const int width = min(P, steps - c0), rows = m - c0;
+  double* Ad = reinterpret_cast<double*>(h.pool) + hm.off + (long long)c0 * m + c0;
+  double* rd = reinterpret_cast<double*>(h.pool) + hm.off + (long long)m * (hm.nj + 1);
+  double* bt = rd + hm.nj + 1;
+  double a[HUB_PANEL_RP][P];
+#pragma unroll
+  for (int k = 0; k < HUB_PANEL_RP; ++k)
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int r = tid + k * HUB_PANEL_THREADS;
+      a[k][i] = (i < width && r < rows) ? Ad[(long long)i * m + r] : 0.0;
+    }
+  if (tid < P * P) T[tid / P][tid % P] = 0.0;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    if (i >= width) break;
+    // products of column i with every column, rows >= i (rows < i: 0 of the first eight threads)
+    double s[P];
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+      s[j] = tid >= i ? a[0][i] * a[0][j] : 0.0;
+#pragma unroll
+      for (int k = 1; k < HUB_PANEL_RP; ++k) s[j] += a[k][i] * a[k][j];
+    }
+    // lane j < P gets the warp's sum of s[j]
+#pragma unroll
+    for (int d = P / 2; d > 0; d >>= 1) {
+      const bool up = lane & d;
+#pragma unroll
+      for (int j = 0; j < d; ++j) {
+        const double give = up ? s[j] : s[j + d], keep = up ? s[j + d] : s[j];
+        s[j] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+      }
+    }
+#pragma unroll
+    for (int d = P; d < 32; d <<= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], d);
+    if (lane < P) red[lane][wid] = s[0];
+    if (tid == i) {
+#pragma unroll
+      for (int j = 0; j < P; ++j) prow[j] = a[0][j];
+    }
+    __syncthreads();
+    if (wid < P) {
+      double t = lane < W ? red[wid][lane] : 0.0;
+#pragma unroll
+      for (int d = W / 2; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
+      if (lane == 0) tot[wid] = t;
+    }
+    __syncthreads();
+    const double x0 = prow[i], nrm = sqrt(tot[i]);
+    double alpha = 0.0, beta = 0.0;
+    if (nrm > 0.0) {
+      alpha = (x0 > 0.0) ? -nrm : nrm;
+      beta = 1.0 / (nrm * (nrm + fabs(x0)));  // 2 / (v^T v)
+      if (tid == i) a[0][i] = x0 - alpha;
+    }
+#pragma unroll
+    for (int j = i + 1; j < P; ++j) {
+      const double w = beta * (tot[j] - alpha * prow[j]);
+      if (tid >= i) a[0][j] -= w * a[0][i];
+#pragma unroll
+      for (int k = 1; k < HUB_PANEL_RP; ++k) a[k][j] -= w * a[k][i];
+    }
+    // T(0 .. i-1, i) = -beta T (V^T v_i), T(i, i) = beta.  Row i of the
+    // reflectors before it is part of v_l: prow[l]
+    if (tid < i) {
+      double t = 0.0;
+      for (int l = tid; l < i; ++l) t += T[tid][l] * (tot[l] - alpha * prow[l]);
+      T[tid][i] = -beta * t;
+    } else if (tid == i) {
+      T[i][i] = beta;
+      rd[c0 + i] = alpha;
+      bt[c0 + i] = beta;
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int k = 0; k < HUB_PANEL_RP; ++k)
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+      const int r = tid + k * HUB_PANEL_THREADS;
+      if (i < width && r < rows) Ad[(long long)i * m + r] = a[k][i];
+    }
+  if (tid < P * P) tq[(long long)blockIdx.x * P * P + tid] = T[tid / P][tid % P];
+}
+
+// a -= V T^T (V^T a) for the trailing columns of every active hub: the panel's
+// reflectors in shared memory, HUB_UP_COLS columns to a warp; pre[g] = blocks of
+// the hubs before g.
+__global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0, int active,
+                                                               const int* __restrict__ pre,
+                                                               const double* __restrict__ tq) {
+  constexpr int P = HUB_PANEL, Q = HUB_UP_COLS;
+  static_assert(P * Q == 32, "a lane to a product");
+  extern __shared__ __align__(16) double hub_v[];  // [rows][P]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int b = blockIdx.x;
+  int lo = 0, hi = active - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pre[mid] <= b) lo = mid;
+    else hi = mid - 1;
+  }
+  const HubMeta hm = h.meta[lo];
+  const int m = hm.m, steps = min(hm.nj, m), rows = m - c0;
+  const int j0 = c0 + min(P, steps - c0) + (b - pre[lo]) * HUB_UP_BLOCK + wid * Q;
+  const double* V = reinterpret_cast<const double*>(h.pool) + hm.off + (long long)c0 * m + c0;
+  double* A = reinterpret_cast<double*>(h.pool) + hm.off + c0;
+  cudaGridDependencySynchronize();  // the panel's reflectors and T
+  if (c0 >= steps) return;
+  const int width = min(P, steps - c0);
+  // (V's rows above a reflector's own hold R: zeros here)
+  for (int i = 0; i < P; ++i)
+    for (int r = tid; r < rows; r += HUB_UP_THREADS) {
+      double* dst = hub_v + (long long)i * rows + r;
+      if (i < width && r >= i)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" : : "r"(smem_u32(dst)), "l"(V + (long long)i * m + r)
+                     : "memory");
+      else
+        *dst = 0.0;
+    }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  if (j0 > hm.nj) return;  // (no barrier follows)
+  double y[P * Q];
+#pragma unroll
+  for (int e = 0; e < P * Q; ++e) y[e] = 0.0;
+  // U rows of the warp's columns in flight at once
+  constexpr int U = 4;
+  for (int r0 = lane; r0 < rows; r0 += 32 * U) {
+    double x[U][Q];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int r = r0 + 32 * u;
+        x[u][q] = (r < rows && j0 + q <= hm.nj) ? A[(long long)(j0 + q) * m + r] : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (r0 + 32 * u >= rows) break;
+#pragma unroll
+      for (int i = 0; i < P; ++i) {
+        const double v = hub_v[(long long)i * rows + r0 + 32 * u];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) y[q * P + i] += v * x[u][q];
+      }
+    }
+  }
+  // lane q * P + i gets the sum of product (i, q)
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    const bool up = lane & d;
+#pragma unroll
+    for (int e = 0; e < d; ++e) {
+      const double give = up ? y[e] : y[e + d], keep = up ? y[e + d] : y[e];
+      y[e] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+    }
+  }
+  const int i = lane & (P - 1);
+  double w = 0.0;
+#pragma unroll
+  for (int l = 0; l < P; ++l) {
+    const double yl = __shfl_sync(0xffffffffu, y[0], (lane & ~(P - 1)) + l);
+    if (l <= i) w += tq[(long long)lo * P * P + l * P + i] * yl;
+  }
+  double wb[P * Q];
+#pragma unroll
+  for (int e = 0; e < P * Q; ++e) wb[e] = __shfl_sync(0xffffffffu, w, e);
+  for (int r0 = lane; r0 < rows; r0 += 32 * U) {
+    double x[U][Q];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int r = r0 + 32 * u;
+        x[u][q] = (r < rows && j0 + q <= hm.nj) ? A[(long long)(j0 + q) * m + r] : 0.0;
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int r = r0 + 32 * u;
+      if (r >= rows) break;
+#pragma unroll
+      for (int k = 0; k < P; ++k) {
+        const double v = hub_v[(long long)k * rows + r];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) x[u][q] -= wb[q * P + k] * v;
+      }
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (j0 + q <= hm.nj) A[(long long)(j0 + q) * m + r] = x[u][q];
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(LG_BLOCK) k_hub_solve(HubArgs h, LargeArgs a) {
   __shared__ T ys[LG_NJ_MAX];
@@ -1957,6 +2183,55 @@ int run_rows_rest(Ctx* c, const SmallArgs& sa, int mid) {
   return launch_rows<T, GroupC>(c, ga);
 }
 
+// The panels of all hubs (sorted by |J| descending): factor, then apply, per panel.
+int hub_panels(Ctx* c, const HubArgs& h, const std::vector<HubMeta>& hm, int steps) {
+  const int nh = (int)hm.size(), np = (steps + HUB_PANEL - 1) / HUB_PANEL;
+  // per panel: active hubs, blocks of the hubs before each, tallest block left
+  std::vector<int> pre((size_t)np * (nh + 1), 0), act(np, 0), tall(np, 1);
+  for (int p = 0; p < np; ++p) {
+    const int c0 = p * HUB_PANEL;
+    int* q = pre.data() + (size_t)p * (nh + 1);
+    for (int g = 0; g < nh; ++g) {
+      const int st = std::min(hm[g].nj, hm[g].m);
+      if (hm[g].nj > c0) act[p] = g + 1;
+      const int cols = st > c0 ? hm[g].nj + 1 - (c0 + std::min(HUB_PANEL, st - c0)) : 0;
+      if (st > c0) tall[p] = std::max(tall[p], hm[g].m - c0);
+      q[g + 1] = q[g] + (cols + HUB_UP_BLOCK - 1) / HUB_UP_BLOCK;
+    }
+  }
+  const size_t tbytes = sizeof(double) * HUB_PANEL * HUB_PANEL * (size_t)nh;
+  DCU_TRY(ensure(c, B_HUBT, tbytes + sizeof(int) * pre.size()));
+  double* tq = bp<double>(c, B_HUBT);
+  int* dpre = reinterpret_cast<int*>(bp<char>(c, B_HUBT) + tbytes);
+  DCU_CUDA(c, cudaMemcpyAsync(dpre, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, c->stream));
+  DCU_CUDA(c, cudaFuncSetAttribute(k_hub_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)(sizeof(double) * HUB_PANEL * HUB_TALL)));
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = c->stream;
+  cfg.attrs = at;
+  for (int p = 0; p < np; ++p) {
+    const int blocks = pre[(size_t)p * (nh + 1) + act[p]];
+    cfg.numAttrs = p > 0 ? 1 : 0;  // the first panel follows copies
+    cfg.gridDim = dim3(act[p]);
+    cfg.blockDim = dim3(HUB_PANEL_THREADS);
+    cfg.dynamicSmemBytes = 0;
+    DCU_CUDA(c, cudaLaunchKernelEx(&cfg, k_hub_panel, h, p * HUB_PANEL, tq));
+    c->launches++;
+    if (blocks == 0) continue;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(HUB_UP_THREADS);
+    cfg.dynamicSmemBytes = sizeof(double) * HUB_PANEL * (size_t)tall[p];
+    DCU_CUDA(c, cudaLaunchKernelEx(&cfg, k_hub_update, h, p * HUB_PANEL, act[p],
+                                   (const int*)(dpre + (size_t)p * (nh + 1)), (const double*)tq));
+    c->launches++;
+  }
+  return DCU_OK;
+}
+
 template <typename T, int MODE>
 int run_large(Ctx* c, LargeArgs& a, int nbig, int cta_max_area = 0) {
   const size_t fixed = ((sizeof(LargeSmem<T>) + 15) / 16) * 16 + LG_STAGE_BYTES;
@@ -2025,6 +2300,16 @@ int run_large(Ctx* c, LargeArgs& a, int nbig, int cta_max_area = 0) {
   DCU_CUDA(c, cudaMemcpyAsync(c->buf[B_HUBWPRE].p, spre.data(), sizeof(int) * spre.size(), cudaMemcpyHostToDevice,
                               c->stream));
   HubArgs h{a.hub_meta, bp<int>(c, B_HUBWPRE), nh, a.hub_pool};
+  if constexpr (std::is_same<T, double>::value) {
+    int tall = 1;
+    for (const HubMeta& g : hm) tall = std::max(tall, g.m);
+    if (tall <= HUB_TALL) {
+      DCU_TRY(hub_panels(c, h, hm, steps));
+      k_hub_solve<T><<<nh, LG_BLOCK, 0, c->stream>>>(h, a);
+      DCU_LAUNCHED(c, "k_hub_solve");
+      return DCU_OK;
+    }
+  }
   int active = nh;
   for (int cst = -1; cst < steps; ++cst) {
     while (active > 0 && hm[active - 1].nj <= cst) --active;  // hubs with nj > cst
@@ -2202,7 +2487,11 @@ int build_finish(Ctx* c, int n, const int* ptr, const int* idx, const double* va
     la.area_per_block = area;
     memcpy(&la.area_sum, reinterpret_cast<long long*>(st) + ST_AREASUM64, sizeof la.area_sum);
     J->finish_launched = true;
-    DCU_TRY((run_large<T, MODE_BUILD>(c, la, nbig, cta_max_area)));
+    const bool v64 = J->opt.precision == DCU_PREC_M_FP32 || J->opt.precision == DCU_PREC_M_BF16;
+    if (std::is_same<T, float>::value && v64 && J->thread_path)
+      DCU_TRY((run_large<double, MODE_BUILD>(c, la, nbig, cta_max_area)));  // (as the hand-offs above)
+    else
+      DCU_TRY((run_large<T, MODE_BUILD>(c, la, nbig, cta_max_area)));
     DCU_TRY(read_stats(c, st));
     if (st[ST_LIMIT] > 0) return fail(c, DCU_ERR_LIMIT, "%d columns exceeded the CTA kernel's limits", st[ST_LIMIT]);
     if (st[ST_STAGE_FAIL] > 0) return fail(c, DCU_ERR_CUDA, "a bulk copy into shared memory did not complete");
