@@ -211,6 +211,7 @@ struct SellPlan {
   // one-launch solver (persist.cu): most slots and most segments of long rows
   // any of its blocks holds; 0 slots when it does not take an operator of this size
   int max_block_slots = 0, max_block_long = 0;
+  long long uniform_slots = 0;  // slots in offset-uniform slices
 };
 
 // How the one-launch solver splits an operator of n rows: `blocks` blocks

@@ -21,7 +21,8 @@
 //   cluster  up to 16 CTAs of one cluster; the gathered vectors are in shared
 //            memory and read through distributed shared memory, the barrier is
 //            the cluster's hardware barrier, partial sums are written into
-//            every CTA's shared memory before it.
+//            every CTA's shared memory before it.  Where the columns are
+//            scattered the rows are written to every CTA and gathered locally.
 //   grid     one block per SM (a cooperative launch); the gathered vectors are
 //            in global memory (L2), the barrier is one tagged slot per block
 //            that every block polls (arrival and partial sums in one, no
@@ -54,6 +55,7 @@ constexpr int kPSlices = 64;        // slices per block, at most (2048 rows)
 constexpr unsigned kPollLimit = 1u << 22;  // polls of one barrier before it gives up (seconds)
 
 enum { P_ERR_TIMEOUT = 1, P_ERR_CAPACITY = 2 };
+enum { P_GRID = 0, P_PULL = 1, P_PUSH = 2 };  // the grid form; the cluster form, gathering from or writing to the others
 
 // One block's partial sums at one barrier: each FP64 value as two words of
 // 32 bits of it and the barrier's number, so that a word that carries the
@@ -112,27 +114,29 @@ __device__ __forceinline__ void p_cluster_barrier() {
 template <typename MT>
 struct PSmem {
   double* a;         // [cap_slots] A's entries
-  double* r;         // cluster form: [rows] r, q, Ay, y / z
+  double* r;         // cluster forms: r, q, Ay, y / z of the block's rows (pull) or of all rows (push)
   double* q;
-  double* ay;
+  double* ay;        // (push: q's array; q is last read before Ay is written)
   double* yz;
   double* lval;      // [cap_long] sums of the long rows' segments
   MT* m;             // [cap_slots] M's entries
-  unsigned* e;       // [cap_slots] column (grid) or shared::cluster address of r[column]
+  unsigned* e;       // [cap_slots] column (pull: shared::cluster address of r[column])
   int* lstart;       // [cap_long] a segment's entries
   int* llen;         // [cap_long]
 };
 
-template <typename MT, bool CL>
-__host__ __device__ inline size_t p_layout(int cap_slots, int cap_long, int rows, PSmem<MT>* s, unsigned char* base) {
+template <typename MT, int FORM>
+__host__ __device__ inline size_t p_layout(int cap_slots, int cap_long, int rows, int n, PSmem<MT>* s,
+                                           unsigned char* base) {
   size_t o = 0;
   auto take = [&](size_t bytes) {
     const size_t at = o;
     o += (bytes + 15) & ~(size_t)15;
     return at;
   };
-  const size_t nr = CL ? (size_t)rows * 8 : 0;
-  const size_t oa = take((size_t)cap_slots * 8), orr = take(nr), oq = take(nr), oy = take(nr), oz = take(nr);
+  const size_t nr = FORM == P_PULL ? (size_t)rows * 8 : FORM == P_PUSH ? (size_t)n * 8 : 0;
+  const size_t oa = take((size_t)cap_slots * 8), orr = take(nr), oq = take(nr);
+  const size_t oy = FORM == P_PUSH ? oq : take(nr), oz = take(nr);
   const size_t ol = take((size_t)cap_long * 8), om = take((size_t)cap_slots * sizeof(MT));
   const size_t oe = take((size_t)cap_slots * 4), os = take((size_t)cap_long * 4), on = take((size_t)cap_long * 4);
   if (s) {
@@ -152,9 +156,10 @@ __host__ __device__ inline size_t p_layout(int cap_slots, int cap_long, int rows
 
 // Rows [32 spb b, 32 spb (b + 1)) belong to block b, row i of them to thread
 // i % PT (PT threads, RPT rows each): a warp holds whole slices, entry k of its 32 rows side by side.
-template <typename MT, int PT, int RPT, bool CL>
+template <typename MT, int PT, int RPT, int FORM>
 __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   constexpr int PW = PT / 32;
+  constexpr bool CL = FORM != P_GRID, PULL = FORM == P_PULL, PUSH = FORM == P_PUSH;
   extern __shared__ __align__(16) unsigned char p_raw[];
   __shared__ int sbase[kPSlices + 1];
   __shared__ int slong[2];                 // segments of long rows, their entries
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   const int bid = blockIdx.x;
   const int rows_pb = a.spb * 32;
   PSmem<MT> S;
-  p_layout<MT, CL>(a.cap_slots, a.cap_long, rows_pb, &S, p_raw);
+  p_layout<MT, FORM>(a.cap_slots, a.cap_long, rows_pb, a.n, &S, p_raw);
   const unsigned base_r = p_smem(S.r);
   const unsigned off_q = p_smem(S.q) - base_r, off_ay = p_smem(S.ay) - base_r, off_yz = p_smem(S.yz) - base_r;
   const int s0 = bid * a.spb, ns = max(0, min(a.spb, a.nslices - s0));
@@ -228,7 +233,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     }
     S.a[dst] = av;
     S.m[dst] = mv;
-    S.e[dst] = CL ? p_mapa(base_r + 8u * (unsigned)(c % rows_pb), (unsigned)(c / rows_pb)) : (unsigned)c;
+    S.e[dst] = PULL ? p_mapa(base_r + 8u * (unsigned)(c % rows_pb), (unsigned)(c / rows_pb)) : (unsigned)c;
   };
   int li[RPT];  // a long row's first segment in lval and their number << 16, or -1
 #pragma unroll
@@ -297,13 +302,16 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   const int nlong = min(slong[0], a.cap_long);
 
   // ---- gathers ------------------------------------------------------------
-  auto g_r = [&](unsigned e) { return CL ? p_ldc(e) : a.rq[e].x; };
-  auto g_ay = [&](unsigned e) { return CL ? p_ldc(e + off_ay) : a.ay[e]; };
-  auto g_yz = [&](unsigned e) { return CL ? p_ldc(e + off_yz) : a.yz[e]; };
+  auto g_r = [&](unsigned e) { return PUSH ? S.r[e] : PULL ? p_ldc(e) : a.rq[e].x; };
+  auto g_ay = [&](unsigned e) { return PUSH ? S.ay[e] : PULL ? p_ldc(e + off_ay) : a.ay[e]; };
+  auto g_yz = [&](unsigned e) { return PUSH ? S.yz[e] : PULL ? p_ldc(e + off_yz) : a.yz[e]; };
   double beta = 0.0, nalpha = 0.0;
   auto x_p = [&](unsigned e) {  // p at a gathered column
     double rv, qv;
-    if (CL) {
+    if (PUSH) {
+      rv = S.r[e];
+      qv = S.q[e];
+    } else if (PULL) {
       rv = p_ldc(e);
       qv = p_ldc(e + off_q);
     } else {
@@ -524,8 +532,16 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   };
 
   // ---- the solve ------------------------------------------------------------
+  // push: this row's value into every CTA's copy of the vector
+  auto push = [&](double* vec, int row, double v) {
+    const unsigned at = p_smem(vec + row);
+    for (int k = 0; k < a.blocks; ++k) p_stc(p_mapa(at, (unsigned)k), v);
+  };
   auto put_rq = [&](int j, double rv, double qv) {
-    if (CL) {
+    if (PUSH) {
+      push(S.r, row_of(j), rv);
+      push(S.q, row_of(j), qv);
+    } else if (PULL) {
       S.r[tid + j * PT] = rv;
       S.q[tid + j * PT] = qv;
     } else {
@@ -533,11 +549,13 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     }
   };
   auto put_ay = [&](int j, double v) {
-    if (CL) S.ay[tid + j * PT] = v;
+    if (PUSH) push(S.ay, row_of(j), v);
+    else if (PULL) S.ay[tid + j * PT] = v;
     else a.ay[row_of(j)] = v;
   };
   auto put_yz = [&](int j, double v) {
-    if (CL) S.yz[tid + j * PT] = v;
+    if (PUSH) push(S.yz, row_of(j), v);
+    else if (PULL) S.yz[tid + j * PT] = v;
     else a.yz[row_of(j)] = v;
   };
   double r[RPT], p[RPT], ay[RPT], x[RPT], y[RPT], z[RPT];
@@ -715,9 +733,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
 }
 
 // *ran stays false when the device cannot hold all the blocks at once.
-template <typename MT, int PT, int RPT, bool CL>
+template <typename MT, int PT, int RPT, int FORM>
 int p_launch(Ctx* c, PArgs& a, size_t smem, bool* ran) {
-  auto kernel = k_bi_persist<MT, PT, RPT, CL>;
+  constexpr bool CL = FORM != P_GRID;
+  auto kernel = k_bi_persist<MT, PT, RPT, FORM>;
   DCU_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(a.blocks);
@@ -755,14 +774,22 @@ int p_launch(Ctx* c, PArgs& a, size_t smem, bool* ran) {
 }
 
 template <typename MT>
-int p_dispatch(Ctx* c, PArgs& a, size_t smem, bool cl, bool* ran) {
+int p_dispatch(Ctx* c, PArgs& a, size_t smem, int form, bool* ran) {
   const int rows = a.spb * 32;
-  if (cl)
-    return rows <= 512 ? p_launch<MT, 512, 1, true>(c, a, smem, ran) : p_launch<MT, 512, 2, true>(c, a, smem, ran);
+  if (form == P_PUSH) return p_launch<MT, 512, 1, P_PUSH>(c, a, smem, ran);
+  if (form == P_PULL)
+    return rows <= 512 ? p_launch<MT, 512, 1, P_PULL>(c, a, smem, ran) : p_launch<MT, 512, 2, P_PULL>(c, a, smem, ran);
   // (1024 threads hold 64 registers each and spill: 512 x 512 took 11.7 against 10.9 ms)
-  if (rows <= 512) return p_launch<MT, 512, 1, false>(c, a, smem, ran);
-  if (rows <= 1024) return p_launch<MT, 512, 2, false>(c, a, smem, ran);
-  return p_launch<MT, 512, 4, false>(c, a, smem, ran);
+  if (rows <= 512) return p_launch<MT, 512, 1, P_GRID>(c, a, smem, ran);
+  if (rows <= 1024) return p_launch<MT, 512, 2, P_GRID>(c, a, smem, ran);
+  return p_launch<MT, 512, 4, P_GRID>(c, a, smem, ran);
+}
+
+template <typename MT>
+size_t p_bytes(int form, int cap_slots, int cap_long, int rows, int n) {
+  return form == P_PUSH   ? p_layout<MT, P_PUSH>(cap_slots, cap_long, rows, n, nullptr, nullptr)
+         : form == P_PULL ? p_layout<MT, P_PULL>(cap_slots, cap_long, rows, n, nullptr, nullptr)
+                          : p_layout<MT, P_GRID>(cap_slots, cap_long, rows, n, nullptr, nullptr);
 }
 
 // Static shared memory of the kernel, rounded up, and the runtime's own.
@@ -799,14 +826,18 @@ int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* m
   a.cap_slots = plan.max_block_slots;
   a.cap_long = plan.max_block_long;
   const int rows = sh.spb * 32;
-  size_t smem;
-  if (mkind == 0)
-    smem = sh.cluster ? p_layout<double, true>(a.cap_slots, a.cap_long, rows, nullptr, nullptr)
-                      : p_layout<double, false>(a.cap_slots, a.cap_long, rows, nullptr, nullptr);
-  else
-    smem = sh.cluster ? p_layout<float, true>(a.cap_slots, a.cap_long, rows, nullptr, nullptr)
-                      : p_layout<float, false>(a.cap_slots, a.cap_long, rows, nullptr, nullptr);
-  if (smem + kPStatic > c->smem_optin) return DCU_OK;
+  auto bytes = [&](int form) {
+    return kPStatic + (mkind == 0 ? p_bytes<double>(form, a.cap_slots, a.cap_long, rows, plan.n)
+                                  : p_bytes<float>(form, a.cap_slots, a.cap_long, rows, plan.n));
+  };
+  // Scattered columns (fewer than half the slots in slices of one offset a
+  // position): a gather of 32 scattered elements through distributed shared
+  // memory goes lane by lane, so each row is written to every CTA instead and
+  // gathered locally, where the whole vectors fit.
+  int form = sh.cluster ? P_PULL : P_GRID;
+  if (sh.cluster && rows <= 512 && 2 * plan.uniform_slots < plan.slots && bytes(P_PUSH) <= c->smem_optin) form = P_PUSH;
+  if (bytes(form) > c->smem_optin) return DCU_OK;
+  const size_t smem = bytes(form) - kPStatic;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t nslot = sh.cluster ? 0 : sizeof(PSlot) * 2 * kPMaxBlocks;
   const size_t vec = al(sizeof(double) * (size_t)plan.n);
@@ -840,7 +871,7 @@ int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* m
   a.maxiter = opt->maxiter > 0 ? opt->maxiter : plan.n;
   a.verify = opt->verify;
   DCU_CUDA(c, cudaMemsetAsync(base, 0, al(sizeof(SolveOut)) + nslot, c->stream));
-  DCU_TRY(mkind == 0 ? p_dispatch<double>(c, a, smem, sh.cluster, ran) : p_dispatch<float>(c, a, smem, sh.cluster, ran));
+  DCU_TRY(mkind == 0 ? p_dispatch<double>(c, a, smem, form, ran) : p_dispatch<float>(c, a, smem, form, ran));
   if (!*ran) return DCU_OK;
   DCU_CUDA(c, cudaEventRecord(c->ev[1], c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(c->pinned, a.out, sizeof(SolveOut), cudaMemcpyDeviceToHost, c->stream));

@@ -714,10 +714,11 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
       rptr, rcol, rperm, n, nslices, off, sidx, sperm, maxdelta, del, kd, su, pst + 1, wide, c->wide_prepass ? 1 : 0,
       kd8, kd8h, cost, ps.blocks > 0 ? ps.spb : 0);
   DCU_LAUNCHED(c, "k_sell_layout");
+  // [0] wide slices, [1] largest delta, [2] check, then uniform slots and the blocks' costs
   int* hcost = reinterpret_cast<int*>(c->pinned) + 4;
-  static_assert(sizeof(int) * (4 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
-  if (ps.blocks > 0)
-    DCU_CUDA(c, cudaMemcpyAsync(hcost, cost, sizeof(int) * 2 * (size_t)ps.blocks, cudaMemcpyDeviceToHost, c->stream));
+  static_assert(sizeof(int) * (6 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
+  DCU_CUDA(c, cudaMemcpyAsync(hcost, pst + 1, sizeof(unsigned long long) * (1 + (size_t)ps.blocks),
+                              cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(c->pinned, wide, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(reinterpret_cast<int*>(c->pinned) + 1, maxdelta, sizeof(int), cudaMemcpyDeviceToHost,
                               c->stream));
@@ -727,6 +728,8 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_CUDA(c, cudaStreamSynchronize(c->stream));
   if (check_out) *check_out = check ? reinterpret_cast<int*>(c->pinned)[2] : 0;
   plan->nwide = *reinterpret_cast<int*>(c->pinned);
+  std::memcpy(&plan->uniform_slots, hcost, sizeof(long long));
+  hcost += 2;
   plan->max_block_slots = plan->max_block_long = 0;
   for (int g = 0; g < ps.blocks; ++g) {
     plan->max_block_slots = std::max(plan->max_block_slots, hcost[2 * g]);
