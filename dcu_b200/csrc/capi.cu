@@ -638,10 +638,7 @@ int dcu_csc_to_csr_d(dcu_spai_ctx* c, int n, int nnz, const int* ptr, const int*
   DCU_TRY(dcu::validate_csc(c, n, nnz, ptr, idx, /*unique_rows=*/false));
   DCU_TRY(dcu::ensure(c, dcu::B_RPERM, sizeof(int) * (size_t)(nnz > 0 ? nnz : 1)));
   int* perm = dcu::bp<int>(c, dcu::B_RPERM);
-  DCU_TRY(dcu::csr_from_csc(c, n, nnz, ptr, idx, rptr, ridx, perm));
-  if (val && rval) DCU_TRY(dcu::csr_values(c, nnz, perm, val, rval));
-  DCU_CUDA(c, cudaStreamSynchronize(c->stream));
-  return DCU_OK;
+  return dcu::csr_from_csc(c, n, nnz, ptr, idx, rptr, ridx, perm, val, val ? rval : nullptr);
 }
 
 int dcu_bicgstab_d(dcu_spai_ctx* c, int n, int nnz, const int* ptr, const int* idx, const double* val,

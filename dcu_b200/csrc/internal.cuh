@@ -242,8 +242,9 @@ int plan_stats(Ctx* c, long long* slots, long long* uniform_slots, long long* wi
 // fails).  unique_rows also refuses a row index repeated inside one column:
 // every SPAI and solver entry point needs distinct (row, column) pairs.
 int validate_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, bool unique_rows = true);
-int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rptr, int* rcol,
-                 int* rperm);
+// CSR of a CSC matrix (with val and rval its values too); the stream is idle on return.
+int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rptr, int* rcol, int* rperm,
+                 const double* val, double* rval);
 int csr_values(Ctx* c, int nnz, const int* rperm, const double* val, double* rval);
 int sell_plan(Ctx* c, int n, int nnz, const int* ptr, const int* idx, SellPlan* plan);
 // SELL-32 layout of the operator whose CSR is (rptr, rcol, rperm).  With

@@ -44,11 +44,12 @@ __global__ void k_row_scatter(const int* __restrict__ ptr, const int* __restrict
 // strictly ascending, bit 2 = some (r, c) has no (c, r).  Any flag sends the
 // conversion to the general count / scatter / sort path, which rewrites all
 // three outputs.  With copies = 0 only rperm is written (the caller reads
-// ptr and idx as the CSR arrays).
+// ptr and idx as the CSR arrays).  (Columns of up to 10 entries side by side:
+// a 9-point mesh of 250000 columns 25.8 -> 19.0 us against 8.)
 __global__ void k_csr_symmetric(const int* __restrict__ ptr, const int* __restrict__ idx, int n,
                                 int* __restrict__ rptr, int* __restrict__ rcol, int* __restrict__ rperm,
                                 int* __restrict__ flag, int copies) {
-  constexpr int kShort = 8;  // columns up to this long search their partners side by side
+  constexpr int kShort = 10; // columns up to this long search their partners side by side
   int bad = 0;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     const int s = ptr[c], e = ptr[c + 1];
@@ -242,7 +243,10 @@ __global__ void __launch_bounds__(512) k_row_sort_long(const int* __restrict__ r
 
 __global__ void k_gather_f64(const int* __restrict__ perm, const double* __restrict__ src, int nnz,
                              double* __restrict__ dst) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) dst[e] = src[perm[e]];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
+    const int p = perm[e];
+    if (p >= 0) dst[e] = src[p];
+  }
 }
 
 // SELL: slice widths (max row length of each 32-row slice), one warp per slice.
@@ -632,15 +636,21 @@ int csr_general(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rpt
 
 }  // namespace
 
-int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rptr, int* rcol, int* rperm) {
+int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rptr, int* rcol, int* rperm,
+                 const double* val, double* rval) {
   if (n > 0 && nnz > 0) {
     int* flag = nullptr;
     DCU_TRY(csr_try_symmetric(c, n, ptr, idx, rptr, rcol, rperm, &flag, true));
+    // the values without waiting for the verdict (a slot without a partner is -1)
+    if (val && rval) DCU_TRY(csr_values(c, nnz, rperm, val, rval));
     DCU_CUDA(c, cudaMemcpyAsync(c->pinned, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     DCU_CUDA(c, cudaStreamSynchronize(c->stream));
     if (*(int*)c->pinned == 0) return DCU_OK;
   }
-  return csr_general(c, n, nnz, ptr, idx, rptr, rcol, rperm);
+  DCU_TRY(csr_general(c, n, nnz, ptr, idx, rptr, rcol, rperm));
+  if (val && rval) DCU_TRY(csr_values(c, nnz, rperm, val, rval));
+  DCU_CUDA(c, cudaStreamSynchronize(c->stream));
+  return DCU_OK;
 }
 
 int sell_plan(Ctx* c, int n, int nnz, const int* ptr, const int* idx, SellPlan* plan) {
