@@ -26,18 +26,20 @@
 //   grid     one block per SM (a cooperative launch); the gathered vectors are
 //            in global memory (L2), the barrier is one tagged slot per block
 //            that every block polls (arrival and partial sums in one, no
-//            atomics), with an iteration limit.
+//            atomics), with an iteration limit; the two barriers without sums
+//            wait only for the blocks whose rows are gathered.
 // Every block sums the same partials in the same order, so all of them take
 // the same decisions without a further exchange, and the result does not
 // depend on timing.
 //
 // Measured on one B200 (whole calls, before -> with this kernel): 64 x 64 grid
-// 1.16 -> 0.42 ms, 96 x 96 forward and backward 8.4 -> 3.2 ms, the circuit-like
-// matrix of 4510 rows 19.3 -> 6.2 ms (its long rows are no longer a serial chain),
-// 256 x 256 4.6 -> 3.2 ms, 512 x 512 adjoint 14.9 -> 9.9 ms.  An iteration is now
-// bound by its five barriers: about 1.0 us a step in the cluster form (hardware
-// barrier 0.45 us, two block-level sums and one remote gather the rest), about
-// 3.5 us in the grid form (two fences and two trips through L2).
+// 1.17 -> 0.40 ms, 96 x 96 forward and backward 8.4 -> 3.0 ms, the circuit-like
+// matrix of 4510 rows 19.2 -> 7.6 ms (its long rows are no longer a serial chain;
+// 5.0 with the faster build), 256 x 256 4.6 -> 2.8 ms, 512 x 512 adjoint 14.9 ->
+// 8.4 ms.  An iteration is now bound by its five barriers: about 1.0 us a step in
+// the cluster form (hardware barrier 0.45 us, two block-level sums and one
+// remote gather the rest), 2.5 to 3.5 us in the grid form (two fences and two
+// trips through L2).
 //
 // Forms with FP32 search vectors are not taken: their iterates follow every
 // rounding of the dot products, which are summed in another order here.
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   __shared__ int sbase[kPSlices + 1];
   __shared__ int slong[2];                 // segments of long rows, their entries
   __shared__ int ticket;                   // next segment to sum
+  __shared__ unsigned from[kPPoll];        // grid form: the blocks whose rows this one gathers
   __shared__ double red[2][PW];
   __shared__ double sums[2];               // grid form: the totals
   __shared__ double part[2][2][16];        // cluster form: [parity][sum][rank]
@@ -184,6 +187,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   // row, and the others set its width.
   if (tid < 2) slong[tid] = 0;
   if (tid == 0) ticket = 0;
+  if (tid < kPPoll) from[tid] = 0u;
   __syncthreads();
   auto slice_len = [&](int s, int w, bool& split) {  // this lane's row length; whether long rows leave the slice
     const int r = s * 32 + lane;
@@ -233,6 +237,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
     }
     S.a[dst] = av;
     S.m[dst] = mv;
+    if (!CL) {
+      const int o = c / rows_pb;
+      if (!(from[o >> 5] >> (o & 31) & 1u)) atomicOr(&from[o >> 5], 1u << (o & 31));
+    }
     S.e[dst] = PULL ? p_mapa(base_r + 8u * (unsigned)(c % rows_pb), (unsigned)(c / rows_pb)) : (unsigned)c;
   };
   int li[RPT];  // a long row's first segment in lval and their number << 16, or -1
@@ -409,7 +417,10 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   // visible to all threads of all blocks after it.
   unsigned ep = 0;
   double tot[2] = {0.0, 0.0};
-  auto sync = [&](int nd, double v0, double v1) -> bool {
+  // near (grid form, nd = 0): wait only for the blocks whose rows this one
+  // gathers.  Nothing they write is overwritten, and no slot reused, before the
+  // next barrier of all blocks: two near ones never follow each other.
+  auto sync = [&](int nd, double v0, double v1, bool near = false) -> bool {
     ++ep;
     const unsigned par = ep & 1u;
     if (nd > 0) {
@@ -485,7 +496,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
 #pragma unroll
         for (int m = 0; m < kPPoll; ++m) {
           tv[0][m] = tv[1][m] = 0.0;
-          if (lane + 32 * m >= a.blocks) got |= 1u << m;
+          if (lane + 32 * m >= a.blocks || (near && !(from[m] >> lane & 1u))) got |= 1u << m;
         }
         do {
 #pragma unroll
@@ -573,7 +584,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
 #pragma unroll
     for (int j = 0; j < RPT; ++j)
       if (mine(j)) put_yz(j, x[j]);
-    if (!sync(0, 0.0, 0.0)) return false;
+    if (!sync(0, 0.0, 0.0, true)) return false;
     rows_dot(S.a, g_yz, v);
     double d0 = 0.0, d1 = 0.0;
     bb = 0.0;
@@ -618,7 +629,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       p[j] = r[j] + beta * qv;
       put_yz(j, y[j]);
     }
-    if (!(ok = sync(0, 0.0, 0.0))) break;
+    if (!(ok = sync(0, 0.0, 0.0, true))) break;
     // Ay, alpha
     double d0 = 0.0, d1 = 0.0;
     rows_dot(S.a, g_yz, ay);
@@ -643,7 +654,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       r[j] = r[j] + nalpha * ay[j];
       put_yz(j, z[j]);
     }
-    if (!(ok = sync(0, 0.0, 0.0))) break;
+    if (!(ok = sync(0, 0.0, 0.0, true))) break;
     // Az, omega
     d0 = d1 = 0.0;
     double az[RPT];
@@ -809,7 +820,9 @@ PersistShape persist_shape(const Ctx* c, int n) {
   } else {
     const int g = std::min(c->sms, kPMaxBlocks);
     s.cluster = false;
-    s.spb = (nslices + g - 1) / g;
+    // 512 rows a block at least: fewer blocks to wait for (256 x 256 grid, 128
+    // against 147 blocks: 3.33 -> 3.14 ms; 150 x 150, 44 against 141: 2.01 -> 1.66)
+    s.spb = std::max(16, (nslices + g - 1) / g);
   }
   // (a cluster's size stays a power of two: its last blocks may hold no rows)
   s.blocks = s.cluster ? k : (nslices + s.spb - 1) / s.spb;
