@@ -778,7 +778,12 @@ int p_launch(Ctx* c, PArgs& a, size_t smem, bool* ran) {
     cudaGetLastError();
     return DCU_OK;
   }
-  DCU_CUDA(c, cudaLaunchKernelEx(&cfg, kernel, a));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, a);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources) {
+    cudaGetLastError();
+    return DCU_OK;
+  }
+  if (e != cudaSuccess) return cuda_fail(c, e, "k_bi_persist", __FILE__, __LINE__);
   c->launches++;
   *ran = true;
   return DCU_OK;
