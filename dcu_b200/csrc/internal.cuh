@@ -223,6 +223,23 @@ struct PersistShape {
 constexpr int kPersistLong = 16;     // a longer row of a wide slice is summed by a warp
 constexpr int kPersistSeg = 128;     // entries of such a row that one warp takes at a time
 constexpr int kPersistBlocks = 160;  // most blocks (a multiple of 32)
+
+// Whether the one-launch solver takes the long rows (over kPersistLong
+// entries) of a slice of w slots out of it, by its lanes' row lengths: when
+// they are few (the rule of the wide pre-pass), or when over three quarters of
+// the slots are padding.  Such a slice is laid out compactly.  Without the
+// second rule a hub row beside five rows of 17 entries (one circuit-like matrix
+// of 4510 rows in eight has such a slice) keeps 32 x 400 slots, more than a
+// block's shared memory, and the solve goes back to five launches an iteration
+// (build and solve 22.7 ms, 4.6 with it).
+#ifdef __CUDACC__
+__device__ __forceinline__ bool slice_split(int w, int len) {
+  static_assert(kPersistLong == kWideSlice, "a slice of the wide pre-pass is one of these");
+  const int nlong = __popc(__ballot_sync(0xffffffffu, len > kWideSlice));
+  const int total = __reduce_add_sync(0xffffffffu, len);
+  return w > kPersistLong && (nlong <= kWideRows || total < 8 * w);
+}
+#endif
 PersistShape persist_shape(const Ctx* c, int n);
 
 // What the one-launch solver writes at its end.

@@ -181,10 +181,9 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   int err = 0;
 
   // ---- the block's entries into shared memory -----------------------------
-  // A slice keeps all its slots, except one made wider than kPLong by at most
-  // kWideRows long rows (laid out compactly: entries in row order, padding at
-  // the end): its rows longer than kPLong go to the long list, a warp to a
-  // row, and the others set its width.
+  // A slice keeps all its slots, except one that slice_split names (laid out
+  // compactly: entries in row order, padding at the end): its rows longer than
+  // kPLong go to the long list, a warp to a row, and the others set its width.
   if (tid < 2) slong[tid] = 0;
   if (tid == 0) ticket = 0;
   if (tid < kPPoll) from[tid] = 0u;
@@ -192,7 +191,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   auto slice_len = [&](int s, int w, bool& split) {  // this lane's row length; whether long rows leave the slice
     const int r = s * 32 + lane;
     const int len = r < a.n ? a.rptr[r + 1] - a.rptr[r] : 0;
-    split = w > kPLong && __popc(__ballot_sync(0xffffffffu, len > kWideSlice)) <= kWideRows;
+    split = slice_split(w, len);
     return len;
   };
   for (int t = wid; t < ns; t += PW) {

@@ -337,12 +337,13 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       sidx[q] = col;
       note(k, q, col);
     }
-    // rows of the slice longer than kWideSlice; where they are few, a row's
-    // sum stops at its own length (wide_row, the one-launch solver's long
-    // rows), which needs its entries in the first slots
-    const int nlong = __popc(__ballot_sync(0xffffffffu, len > kWideSlice));
-    const bool few_long = w > kWideSlice && nlong <= kWideRows;
-    if (!__all_sync(0xffffffffu, i == len) || few_long) {
+    // rows of the slice longer than kWideSlice; where they are few, or the
+    // slice is mostly padding, a row's sum stops at its own length (wide_row,
+    // the one-launch solver's long rows), which needs its entries in the first
+    // slots
+    const bool few_long = w > kWideSlice && __popc(__ballot_sync(0xffffffffu, len > kWideSlice)) <= kWideRows;
+    const bool sparse = slice_split(w, len);
+    if (!__all_sync(0xffffffffu, i == len) || sparse) {
       all = true;
       my_d = 0;
       for (int k = 0; k < w; ++k) {
@@ -368,7 +369,7 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
     // the slice's share of a block of the one-launch solver (persist.cu, which
     // makes the same split): slots kept, entries and segments of the long rows
     if (spb > 0) {
-      const bool split = w > kPersistLong && few_long;
+      const bool split = sparse;
       const int ws = __reduce_max_sync(0xffffffffu, !split ? w : (len <= kPersistLong ? len : 0));
       const int le = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? len : 0);
       const int nl = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? (len + kPersistSeg - 1) / kPersistSeg : 0);
