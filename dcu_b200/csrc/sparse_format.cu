@@ -22,16 +22,34 @@ __global__ void k_row_count(const int* __restrict__ idx, int nnz, int* __restric
     atomicAdd(&cnt[idx[e]], 1);
 }
 
+// Columns longer than this (hubs of a circuit matrix) are shared by their warp
+// in the passes that otherwise give a column to a thread, where a column of 400
+// entries is 400 dependent steps (circuit-like matrix of 4510 rows: the
+// symmetry check 157 -> 28 us, the scatter 132 -> 18; with the rows of 17 to 64
+// sorted by warps 92 -> 10 and slices that end up compact laid out once 118 -> 43,
+// the whole solve 4.54 -> 4.01 ms).
+constexpr int kCoopLen = 64;
+
 // One thread per column: scatter the column's entries into their rows' slots.
+// The order inside a row is the sort's business (by column, then slot).
 __global__ void k_row_scatter(const int* __restrict__ ptr, const int* __restrict__ idx, int n,
                               const int* __restrict__ rptr, int* __restrict__ fill,
                               int* __restrict__ rcol, int* __restrict__ rperm) {
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-    for (int e = ptr[c]; e < ptr[c + 1]; ++e) {
-      int r = idx[e];
-      int pos = rptr[r] + atomicAdd(&fill[r], 1);
-      rcol[pos] = c;
-      rperm[pos] = e;
+  const int lane = threadIdx.x & 31;
+  auto place = [&](int c, int e) {
+    const int r = idx[e];
+    const int pos = rptr[r] + atomicAdd(&fill[r], 1);
+    rcol[pos] = c;
+    rperm[pos] = e;
+  };
+  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c - lane < n; c += gridDim.x * blockDim.x) {
+    const int s = c < n ? ptr[c] : 0, e = c < n ? ptr[c + 1] : 0;
+    if (e - s <= kCoopLen)
+      for (int k = s; k < e; ++k) place(c, k);
+    for (unsigned longs = __ballot_sync(0xffffffffu, e - s > kCoopLen); longs; longs &= longs - 1) {
+      const int j = __ffs(longs) - 1;
+      const int cs = __shfl_sync(0xffffffffu, s, j), ce = __shfl_sync(0xffffffffu, e, j);
+      for (int k = cs + lane; k < ce; k += 32) place(c - lane + j, k);
     }
   }
 }
@@ -50,7 +68,21 @@ __global__ void k_csr_symmetric(const int* __restrict__ ptr, const int* __restri
                                 int* __restrict__ rptr, int* __restrict__ rcol, int* __restrict__ rperm,
                                 int* __restrict__ flag, int copies) {
   constexpr int kShort = 10; // columns up to this long search their partners side by side
+  const int lane = threadIdx.x & 31;
   int bad = 0;
+  // entry k (row r) of column c: its place among column r's entries
+  auto partner = [&](int c, int r) {
+    int lo = ptr[r], hi = ptr[r + 1] - 1;
+    while (lo <= hi) {
+      const int mid = (lo + hi) >> 1;
+      const int v = idx[mid];
+      if (v == c) return mid;
+      if (v < c) lo = mid + 1;
+      else hi = mid - 1;
+    }
+    return -1;
+  };
+  bool longs = false;
   for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
     const int s = ptr[c], e = ptr[c + 1];
     if (copies) {
@@ -103,44 +135,83 @@ __global__ void k_csr_symmetric(const int* __restrict__ ptr, const int* __restri
         }
       continue;
     }
+    if (e - s > kCoopLen) {
+      longs = true;
+      continue;
+    }
     int prev = -1;
     for (int k = s; k < e; ++k) {
       const int r = idx[k];
       if (copies) rcol[k] = r;
       if (r <= prev) bad |= 1;
       prev = r;
-      int lo = ptr[r], hi = ptr[r + 1] - 1, q = -1;
-      while (lo <= hi) {
-        const int mid = (lo + hi) >> 1;
-        const int v = idx[mid];
-        if (v == c) {
-          q = mid;
-          break;
-        }
-        if (v < c) lo = mid + 1;
-        else hi = mid - 1;
-      }
+      const int q = partner(c, r);
       if (q < 0) bad |= 2;
       rperm[k] = q;
+    }
+  }
+  // the long columns of the warp's, apart: in the loop above their collectives
+  // cost the others (9-point mesh of 250000 columns, whole call 86.9 -> 95.0 us)
+  if (__any_sync(0xffffffffu, longs)) {
+    for (int c0 = blockIdx.x * blockDim.x + threadIdx.x - lane; c0 < n; c0 += gridDim.x * blockDim.x) {
+      const int c = c0 + lane;
+      const int s = c < n ? ptr[c] : 0, e = c < n ? ptr[c + 1] : 0;
+      for (unsigned m = __ballot_sync(0xffffffffu, e - s > kCoopLen); m; m &= m - 1) {
+        const int j = __ffs(m) - 1;
+        const int cs = __shfl_sync(0xffffffffu, s, j), ce = __shfl_sync(0xffffffffu, e, j);
+        for (int k = cs + lane; k < ce; k += 32) {
+          const int r = idx[k];
+          if (copies) rcol[k] = r;
+          if (r <= (k > cs ? idx[k - 1] : -1)) bad |= 1;
+          const int q = partner(c0 + j, r);
+          if (q < 0) bad |= 2;
+          rperm[k] = q;
+        }
+      }
     }
   }
   if (__any_sync(0xffffffffu, bad != 0) && bad) atomicOr(flag, bad);
 }
 
 constexpr int kRegSortMax = 16;     // rows sorted in registers by one thread
-constexpr int kThreadSortMax = 64;  // rows sorted in place by one thread
+constexpr int kThreadSortMax = 64;  // rows sorted by one warp
 
 // Rows up to kRegSortMax entries: loaded into registers as (col << 32 | slot)
 // keys, sorted with a static insertion network, written back only when out
-// of order.  Rows up to kThreadSortMax: insertion sort in place.  Longer rows
-// are queued for the block sort.  Column indices inside a row are distinct
-// (a CSC column lists each row once), so the order is unique.
+// of order.  Rows up to kThreadSortMax: one after another by the warp, each
+// entry put at the place its key has among the row's.  Longer rows are queued
+// for the block sort.  The slots are distinct, so the order is unique also
+// where a column lists a row twice.
 __global__ void k_row_sort_short(const int* __restrict__ rptr, int n, int* __restrict__ rcol,
                                  int* __restrict__ rperm, int* __restrict__ long_rows,
                                  int* __restrict__ long_count) {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    const int s = rptr[r], e = rptr[r + 1];
+  static_assert(kThreadSortMax <= 64, "two keys a lane");
+  const int lane = threadIdx.x & 31;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r - lane < n; r += gridDim.x * blockDim.x) {
+    const int s = r < n ? rptr[r] : 0, e = r < n ? rptr[r + 1] : 0;
     const int len = e - s;
+    for (unsigned mid = __ballot_sync(0xffffffffu, len > kRegSortMax && len <= kThreadSortMax); mid; mid &= mid - 1) {
+      const int j = __ffs(mid) - 1;
+      const int ms = __shfl_sync(0xffffffffu, s, j), ml = __shfl_sync(0xffffffffu, len, j);
+      unsigned long long key[2];
+      int at[2] = {0, 0};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        key[h] = i < ml ? ((unsigned long long)(unsigned)rcol[ms + i] << 32) | (unsigned)rperm[ms + i] : ~0ull;
+      }
+      for (int i = 0; i < ml; ++i) {
+        const unsigned long long k = __shfl_sync(0xffffffffu, i < 32 ? key[0] : key[1], i & 31);
+        at[0] += k < key[0];
+        at[1] += k < key[1];
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (lane + 32 * h < ml) {
+          rcol[ms + at[h]] = (int)(key[h] >> 32);
+          rperm[ms + at[h]] = (int)(key[h] & 0xffffffffu);
+        }
+    }
     if (len <= kRegSortMax) {
       unsigned long long key[kRegSortMax];
       bool sorted = true;
@@ -178,18 +249,6 @@ __global__ void k_row_sort_short(const int* __restrict__ rptr, int n, int* __res
     if (len > kThreadSortMax) {
       long_rows[atomicAdd(long_count, 1)] = r;
       atomicMax(long_count + 1, len);
-      continue;
-    }
-    for (int i = s + 1; i < e; ++i) {
-      int kc = rcol[i], kp = rperm[i];
-      int j = i - 1;
-      while (j >= s && rcol[j] > kc) {
-        rcol[j + 1] = rcol[j];
-        rperm[j + 1] = rperm[j];
-        --j;
-      }
-      rcol[j + 1] = kc;
-      rperm[j + 1] = kp;
     }
   }
 }
@@ -319,8 +378,14 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       if (lane == 0) kd[(o0 >> 5) + k] = same ? (int)(((unsigned)d0 << 1) | 1u) : 0;
       if (lane == k) my_d = d0;
     };
+    // rows of the slice longer than kWideSlice: where they are few, or the
+    // slice is mostly padding, a row's sum stops at its own length (wide_row,
+    // the one-launch solver's long rows), which needs its entries in the first
+    // slots
+    const bool few_long = w > kWideSlice && __popc(__ballot_sync(0xffffffffu, len > kWideSlice)) <= kWideRows;
+    const bool sparse = slice_split(w, len);
     int i = 0;
-    for (int k = 0; k < w; ++k) {
+    for (int k = 0; k < (sparse ? 0 : w); ++k) {
       const int cand = (i < len) ? rcol[rs + i] - r : INT_MAX;
       const int m = __reduce_min_sync(0xffffffffu, cand);
       const long long q = base + 32ll * k;
@@ -337,13 +402,7 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       sidx[q] = col;
       note(k, q, col);
     }
-    // rows of the slice longer than kWideSlice; where they are few, or the
-    // slice is mostly padding, a row's sum stops at its own length (wide_row,
-    // the one-launch solver's long rows), which needs its entries in the first
-    // slots
-    const bool few_long = w > kWideSlice && __popc(__ballot_sync(0xffffffffu, len > kWideSlice)) <= kWideRows;
-    const bool sparse = slice_split(w, len);
-    if (!__all_sync(0xffffffffu, i == len) || sparse) {
+    if (sparse || !__all_sync(0xffffffffu, i == len)) {
       all = true;
       my_d = 0;
       for (int k = 0; k < w; ++k) {
