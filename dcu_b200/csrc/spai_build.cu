@@ -11,8 +11,10 @@
 //                                                     Householder QR of [At | e_E])
 //   M(J_k, k) = m_k                                  (modifyData4_SSPAIv10 :1135-1152)
 //
-// Two kernels share the column range through a device work queue:
-//   k_spai_small  one 16-lane group per column (two per warp), |J_k| <= 7,
+// Kernels share the column range through device work queues:
+//   k_spai_rows   FP64 builds, 4, 8 or 16 lanes per column with its rows spread
+//                 over them, in three sizes up to |J_k| <= 15, |I_k| <= 64.
+//   k_spai_small  FP32 builds and the pattern, one 16-lane group per column (two per warp), |J_k| <= 7,
 //                 <= 64 candidate rows, |I_k| <= 32 (or the tuned
 //                 group_max_ni below it): candidates sorted in registers
 //                 (bitonic network across the group), At staged in shared
@@ -22,7 +24,8 @@
 //                 over the candidate row range, At in shared memory or a
 //                 global slab, Householder with warp-per-trailing-column
 //                 updates, column-oriented back substitution.
-// Columns that do not fit the small kernel are appended to a list the large
+//   k_hub_*       blocks larger than shared memory, on every SM.
+// Columns that do not fit a group kernel are appended to a list the large
 // kernel drains with an atomic counter.  Each column's arithmetic is fixed by
 // its own data (fixed reduction trees, no float atomics), so M is identical
 // for every schedule and grid size.
@@ -337,9 +340,9 @@ __device__ __forceinline__ int group_column(const SmallArgs& a, WarpSmem<T>& ws,
 }
 
 // Held to 80 registers (12 blocks, 24 warps per SM): the Householder steps are
-// latency-bound, and at the unbounded 128 registers only 8 blocks fit (FP64
-// build at 128^3: 7.06 -> 5.92 ms, M bit-identical; at 64 registers it spills
-// and takes 6.3 ms).
+// latency-bound, and at the unbounded 128 registers only 8 blocks fit (128^3 in
+// FP64, which k_spai_rows now builds: 7.06 -> 5.92 ms, M bit-identical; at 64
+// registers it spills and takes 6.3 ms).
 template <typename T, int MODE>
 __global__ void __launch_bounds__(SG_BLOCK, 12) k_spai_small(SmallArgs a) {
   __shared__ WarpSmem<T> smem[SG_WARPS];
