@@ -1806,7 +1806,7 @@ constexpr int HUB_PANEL_THREADS = 512;
 constexpr int HUB_PANEL_RP = 4;       // rows per thread of the panel kernel
 constexpr int HUB_TALL = HUB_PANEL_THREADS * HUB_PANEL_RP;  // tallest block taken by panels
 constexpr int HUB_UP_THREADS = 256;
-constexpr int HUB_UP_COLS = 4;        // trailing columns per warp
+constexpr int HUB_UP_COLS = 2;        // trailing columns per warp
 constexpr int HUB_UP_BLOCK = HUB_UP_COLS * HUB_UP_THREADS / 32;
 
 // Householder factorisation of columns c0 .. c0 + width - 1 of every active hub
@@ -1916,7 +1916,7 @@ __global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0
                                                                const int* __restrict__ pre,
                                                                const double* __restrict__ tq) {
   constexpr int P = HUB_PANEL, Q = HUB_UP_COLS;
-  static_assert(P * Q == 32, "a lane to a product");
+  static_assert(P * Q <= 32 && 32 % (P * Q) == 0, "a lane to a product");
   extern __shared__ __align__(16) double hub_v[];  // [rows][P]
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int b = blockIdx.x;
@@ -1972,9 +1972,13 @@ __global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0
       }
     }
   }
-  // lane q * P + i gets the sum of product (i, q)
+  // the lanes that are q * P + i modulo P * Q get the sum of product (i, q)
 #pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
+  for (int d = 16; d >= P * Q; d >>= 1)
+#pragma unroll
+    for (int e = 0; e < P * Q; ++e) y[e] += __shfl_xor_sync(0xffffffffu, y[e], d);
+#pragma unroll
+  for (int d = P * Q / 2; d > 0; d >>= 1) {
     const bool up = lane & d;
 #pragma unroll
     for (int e = 0; e < d; ++e) {
