@@ -1798,30 +1798,32 @@ __global__ void __launch_bounds__(HUB_THREADS) k_hub_step(HubArgs h, int c, int 
 // Here a panel of up to HUB_PANEL columns is factored by one CTA per hub, with
 // the triangular factor T of its block reflector I - V T V^T, and one launch
 // applies it to all trailing columns: a column crosses L2 once per panel, and
-// two launches replace eight.
+// one launch replaces eight.  The launch's first CTA of each hub takes the next
+// panel's columns and factors them at once, beside the others' updates (whole
+// solve of that matrix 3.98 -> 3.58 ms against two launches a panel).  A step is
+// bound by the leading CTA's chain: V into shared memory, 8 columns updated, 8
+// dependent reductions.
 // The forms with FP32 vectors keep the FP32 steps: their iterates follow every
 // rounding of M.
 constexpr int HUB_PANEL = 8;
 constexpr int HUB_PANEL_THREADS = 512;
 constexpr int HUB_PANEL_RP = 4;       // rows per thread of the panel kernel
 constexpr int HUB_TALL = HUB_PANEL_THREADS * HUB_PANEL_RP;  // tallest block taken by panels
-constexpr int HUB_UP_THREADS = 256;
+constexpr int HUB_UP_THREADS = HUB_PANEL_THREADS;
 constexpr int HUB_UP_COLS = 2;        // trailing columns per warp
 constexpr int HUB_UP_BLOCK = HUB_UP_COLS * HUB_UP_THREADS / 32;
 
-// Householder factorisation of columns c0 .. c0 + width - 1 of every active hub
-// (one block per hub), rows c0 on, in registers: a thread holds HUB_PANEL_RP
+// Householder factorisation of columns c0 .. c0 + width - 1 of a hub by one
+// block, rows c0 on, in registers: a thread holds HUB_PANEL_RP
 // rows of all the panel's columns.  A step takes one block reduction: the
 // column's products with itself, with the columns after it and with the
 // reflectors before it (v = a - alpha e_c, so v^T a_j = a^T a_j - alpha a_j[c]).
-// tq: HUB_PANEL^2 per hub, T by rows.
-__global__ void __launch_bounds__(HUB_PANEL_THREADS) k_hub_panel(HubArgs h, int c0, double* __restrict__ tq) {
+// tq: HUB_PANEL^2, T by rows.
+__device__ __forceinline__ void hub_panel(const HubArgs& h, const HubMeta& hm, int c0, double* __restrict__ tq) {
   constexpr int P = HUB_PANEL, W = HUB_PANEL_THREADS / 32;
   __shared__ double red[P][W + 1], tot[P], prow[P], T[P][P];
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const HubMeta hm = h.meta[blockIdx.x];
   const int m = hm.m, steps = min(hm.nj, m);
-  cudaGridDependencySynchronize();
   if (c0 >= steps) return;
   const int width = min(P, steps - c0), rows = m - c0;
   double* Ad = reinterpret_cast<double*>(h.pool) + hm.off + (long long)c0 * m + c0;
@@ -1906,21 +1908,29 @@ __global__ void __launch_bounds__(HUB_PANEL_THREADS) k_hub_panel(HubArgs h, int 
       const int r = tid + k * HUB_PANEL_THREADS;
       if (i < width && r < rows) Ad[(long long)i * m + r] = a[k][i];
     }
-  if (tid < P * P) tq[(long long)blockIdx.x * P * P + tid] = T[tid / P][tid % P];
+  if (tid < P * P) tq[tid] = T[tid / P][tid % P];
+}
+
+// The first panel of every hub.
+__global__ void __launch_bounds__(HUB_PANEL_THREADS) k_hub_panel(HubArgs h, double* __restrict__ tq) {
+  hub_panel(h, h.meta[blockIdx.x], 0, tq + (long long)blockIdx.x * HUB_PANEL * HUB_PANEL);
 }
 
 // a -= V T^T (V^T a) for the trailing columns of every active hub: the panel's
-// reflectors in shared memory, HUB_UP_COLS columns to a warp; pre[g] = blocks of
-// the hubs before g.
+// reflectors in shared memory, HUB_UP_COLS columns to a warp.  Block g < active
+// takes hub g's next panel and factors it (T to tq_next); the blocks after
+// those take the columns behind it, pre[g] = blocks of the hubs before g.
 __global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0, int active,
                                                                const int* __restrict__ pre,
-                                                               const double* __restrict__ tq) {
+                                                               const double* __restrict__ tq,
+                                                               double* __restrict__ tq_next) {
   constexpr int P = HUB_PANEL, Q = HUB_UP_COLS;
   static_assert(P * Q <= 32 && 32 % (P * Q) == 0, "a lane to a product");
   extern __shared__ __align__(16) double hub_v[];  // [rows][P]
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int b = blockIdx.x;
-  int lo = 0, hi = active - 1;
+  const bool lead = blockIdx.x < active;
+  const int b = blockIdx.x - active;
+  int lo = lead ? blockIdx.x : 0, hi = lead ? lo : active - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (pre[mid] <= b) lo = mid;
@@ -1928,11 +1938,15 @@ __global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0
   }
   const HubMeta hm = h.meta[lo];
   const int m = hm.m, steps = min(hm.nj, m), rows = m - c0;
-  const int j0 = c0 + min(P, steps - c0) + (b - pre[lo]) * HUB_UP_BLOCK + wid * Q;
+  // this block's columns: j_lo .. j_hi - 1
+  const int next = c0 + P, width_next = max(0, min(P, steps - next));
+  const int j_lo = lead ? next : min(next, steps) + width_next + (b - pre[lo]) * HUB_UP_BLOCK;
+  const int j_hi = lead ? next + width_next : hm.nj + 1;
+  const int j0 = j_lo + wid * Q;
   const double* V = reinterpret_cast<const double*>(h.pool) + hm.off + (long long)c0 * m + c0;
   double* A = reinterpret_cast<double*>(h.pool) + hm.off + c0;
   cudaGridDependencySynchronize();  // the panel's reflectors and T
-  if (c0 >= steps) return;
+  if (c0 >= steps || j_lo >= j_hi) return;
   const int width = min(P, steps - c0);
   // (V's rows above a reflector's own hold R: zeros here)
   for (int i = 0; i < P; ++i)
@@ -1946,80 +1960,84 @@ __global__ void __launch_bounds__(HUB_UP_THREADS) k_hub_update(HubArgs h, int c0
     }
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  if (j0 > hm.nj) return;  // (no barrier follows)
-  double y[P * Q];
+  if (j0 < j_hi) {
+    double y[P * Q];
 #pragma unroll
-  for (int e = 0; e < P * Q; ++e) y[e] = 0.0;
-  // U rows of the warp's columns in flight at once
-  constexpr int U = 4;
-  for (int r0 = lane; r0 < rows; r0 += 32 * U) {
-    double x[U][Q];
+    for (int e = 0; e < P * Q; ++e) y[e] = 0.0;
+    // U rows of the warp's columns in flight at once
+    constexpr int U = 4;
+    for (int r0 = lane; r0 < rows; r0 += 32 * U) {
+      double x[U][Q];
 #pragma unroll
-    for (int u = 0; u < U; ++u)
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
+        for (int q = 0; q < Q; ++q) {
+          const int r = r0 + 32 * u;
+          x[u][q] = (r < rows && j0 + q < j_hi) ? A[(long long)(j0 + q) * m + r] : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (r0 + 32 * u >= rows) break;
+#pragma unroll
+        for (int i = 0; i < P; ++i) {
+          const double v = hub_v[(long long)i * rows + r0 + 32 * u];
+#pragma unroll
+          for (int q = 0; q < Q; ++q) y[q * P + i] += v * x[u][q];
+        }
+      }
+    }
+    // the lanes that are q * P + i modulo P * Q get the sum of product (i, q)
+#pragma unroll
+    for (int d = 16; d >= P * Q; d >>= 1)
+#pragma unroll
+      for (int e = 0; e < P * Q; ++e) y[e] += __shfl_xor_sync(0xffffffffu, y[e], d);
+#pragma unroll
+    for (int d = P * Q / 2; d > 0; d >>= 1) {
+      const bool up = lane & d;
+#pragma unroll
+      for (int e = 0; e < d; ++e) {
+        const double give = up ? y[e] : y[e + d], keep = up ? y[e + d] : y[e];
+        y[e] = keep + __shfl_xor_sync(0xffffffffu, give, d);
+      }
+    }
+    const int i = lane & (P - 1);
+    double w = 0.0;
+#pragma unroll
+    for (int l = 0; l < P; ++l) {
+      const double yl = __shfl_sync(0xffffffffu, y[0], (lane & ~(P - 1)) + l);
+      if (l <= i) w += tq[(long long)lo * P * P + l * P + i] * yl;
+    }
+    double wb[P * Q];
+#pragma unroll
+    for (int e = 0; e < P * Q; ++e) wb[e] = __shfl_sync(0xffffffffu, w, e);
+    for (int r0 = lane; r0 < rows; r0 += 32 * U) {
+      double x[U][Q];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int r = r0 + 32 * u;
+          x[u][q] = (r < rows && j0 + q < j_hi) ? A[(long long)(j0 + q) * m + r] : 0.0;
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
         const int r = r0 + 32 * u;
-        x[u][q] = (r < rows && j0 + q <= hm.nj) ? A[(long long)(j0 + q) * m + r] : 0.0;
-      }
+        if (r >= rows) break;
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      if (r0 + 32 * u >= rows) break;
+        for (int k = 0; k < P; ++k) {
+          const double v = hub_v[(long long)k * rows + r];
 #pragma unroll
-      for (int i = 0; i < P; ++i) {
-        const double v = hub_v[(long long)i * rows + r0 + 32 * u];
+          for (int q = 0; q < Q; ++q) x[u][q] -= wb[q * P + k] * v;
+        }
 #pragma unroll
-        for (int q = 0; q < Q; ++q) y[q * P + i] += v * x[u][q];
+        for (int q = 0; q < Q; ++q)
+          if (j0 + q < j_hi) A[(long long)(j0 + q) * m + r] = x[u][q];
       }
     }
   }
-  // the lanes that are q * P + i modulo P * Q get the sum of product (i, q)
-#pragma unroll
-  for (int d = 16; d >= P * Q; d >>= 1)
-#pragma unroll
-    for (int e = 0; e < P * Q; ++e) y[e] += __shfl_xor_sync(0xffffffffu, y[e], d);
-#pragma unroll
-  for (int d = P * Q / 2; d > 0; d >>= 1) {
-    const bool up = lane & d;
-#pragma unroll
-    for (int e = 0; e < d; ++e) {
-      const double give = up ? y[e] : y[e + d], keep = up ? y[e + d] : y[e];
-      y[e] = keep + __shfl_xor_sync(0xffffffffu, give, d);
-    }
-  }
-  const int i = lane & (P - 1);
-  double w = 0.0;
-#pragma unroll
-  for (int l = 0; l < P; ++l) {
-    const double yl = __shfl_sync(0xffffffffu, y[0], (lane & ~(P - 1)) + l);
-    if (l <= i) w += tq[(long long)lo * P * P + l * P + i] * yl;
-  }
-  double wb[P * Q];
-#pragma unroll
-  for (int e = 0; e < P * Q; ++e) wb[e] = __shfl_sync(0xffffffffu, w, e);
-  for (int r0 = lane; r0 < rows; r0 += 32 * U) {
-    double x[U][Q];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        const int r = r0 + 32 * u;
-        x[u][q] = (r < rows && j0 + q <= hm.nj) ? A[(long long)(j0 + q) * m + r] : 0.0;
-      }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int r = r0 + 32 * u;
-      if (r >= rows) break;
-#pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const double v = hub_v[(long long)k * rows + r];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) x[u][q] -= wb[q * P + k] * v;
-      }
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        if (j0 + q <= hm.nj) A[(long long)(j0 + q) * m + r] = x[u][q];
-    }
-  }
+  if (!lead) return;
+  __syncthreads();
+  hub_panel(h, hm, next, tq_next + (long long)lo * P * P);
 }
 
 template <typename T>
@@ -2201,12 +2219,13 @@ int hub_panels(Ctx* c, const HubArgs& h, const std::vector<HubMeta>& hm, int ste
     for (int g = 0; g < nh; ++g) {
       const int st = std::min(hm[g].nj, hm[g].m);
       if (hm[g].nj > c0) act[p] = g + 1;
-      const int cols = st > c0 ? hm[g].nj + 1 - (c0 + std::min(HUB_PANEL, st - c0)) : 0;
+      const int cols = st > c0 ? hm[g].nj + 1 - std::min(c0 + 2 * HUB_PANEL, st) : 0;
       if (st > c0) tall[p] = std::max(tall[p], hm[g].m - c0);
       q[g + 1] = q[g] + (cols + HUB_UP_BLOCK - 1) / HUB_UP_BLOCK;
     }
   }
-  const size_t tbytes = sizeof(double) * HUB_PANEL * HUB_PANEL * (size_t)nh;
+  const size_t tcount = (size_t)HUB_PANEL * HUB_PANEL * nh;
+  const size_t tbytes = 2 * sizeof(double) * tcount;  // T of this panel and of the next one
   DCU_TRY(ensure(c, B_HUBT, tbytes + sizeof(int) * pre.size()));
   double* tq = bp<double>(c, B_HUBT);
   int* dpre = reinterpret_cast<int*>(bp<char>(c, B_HUBT) + tbytes);
@@ -2219,21 +2238,19 @@ int hub_panels(Ctx* c, const HubArgs& h, const std::vector<HubMeta>& hm, int ste
   cudaLaunchConfig_t cfg = {};
   cfg.stream = c->stream;
   cfg.attrs = at;
+  // (the first panel follows copies: no early start)
+  cfg.gridDim = dim3(nh);
+  cfg.blockDim = dim3(HUB_PANEL_THREADS);
+  DCU_CUDA(c, cudaLaunchKernelEx(&cfg, k_hub_panel, h, tq));
+  c->launches++;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(HUB_UP_THREADS);
   for (int p = 0; p < np; ++p) {
-    const int blocks = pre[(size_t)p * (nh + 1) + act[p]];
-    cfg.numAttrs = p > 0 ? 1 : 0;  // the first panel follows copies
-    cfg.gridDim = dim3(act[p]);
-    cfg.blockDim = dim3(HUB_PANEL_THREADS);
-    cfg.dynamicSmemBytes = 0;
-    DCU_CUDA(c, cudaLaunchKernelEx(&cfg, k_hub_panel, h, p * HUB_PANEL, tq));
-    c->launches++;
-    if (blocks == 0) continue;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(HUB_UP_THREADS);
+    cfg.gridDim = dim3(act[p] + pre[(size_t)p * (nh + 1) + act[p]]);
     cfg.dynamicSmemBytes = sizeof(double) * HUB_PANEL * (size_t)tall[p];
     DCU_CUDA(c, cudaLaunchKernelEx(&cfg, k_hub_update, h, p * HUB_PANEL, act[p],
-                                   (const int*)(dpre + (size_t)p * (nh + 1)), (const double*)tq));
+                                   (const int*)(dpre + (size_t)p * (nh + 1)), (const double*)(tq + (p & 1) * tcount),
+                                   tq + ((p + 1) & 1) * tcount));
     c->launches++;
   }
   return DCU_OK;
