@@ -35,8 +35,8 @@
 // Measured on one B200 (whole calls, before -> with this kernel): 64 x 64 grid
 // 1.17 -> 0.40 ms, 96 x 96 forward and backward 8.4 -> 3.0 ms, the circuit-like
 // matrix of 4510 rows 19.2 -> 7.6 ms (its long rows are no longer a serial chain;
-// 4.0 with the faster build and analysis), 256 x 256 4.6 -> 2.8 ms, 512 x 512 adjoint 14.9 ->
-// 8.4 ms.  An iteration is now bound by its five barriers: about 1.0 us a step in
+// 3.5 with the faster build and analysis), 256 x 256 4.6 -> 2.8 ms, 512 x 512 adjoint 14.9 ->
+// 7.8 ms.  An iteration is now bound by its five barriers: about 1.0 us a step in
 // the cluster form (hardware barrier 0.45 us, two block-level sums and one
 // remote gather the rest), 2.5 to 3.5 us in the grid form (two fences and two
 // trips through L2).
