@@ -52,6 +52,14 @@ namespace {
 
 constexpr int kPMaxBlocks = kPersistBlocks;  // grid form
 constexpr int kPPoll = kPMaxBlocks / 32;     // slots a lane polls
+// Grid form: barrier e uses the slots of set e % kPSlotSets.  A block stores
+// its tag over the one of barrier e - kPSlotSets, which every block that polls
+// for it must have seen: a barrier of all blocks has to lie strictly between
+// the two.  Near barriers wait for some blocks only and never follow each
+// other, so of two barriers in a row one is of all blocks: three sets suffice
+// (with two, a block past a near barrier may overwrite a tag that a distant
+// block still polls for), four make the set a mask.
+constexpr int kPSlotSets = 4;
 constexpr int kPLong = kPersistLong;  // a longer row of a wide slice is summed by a warp
 constexpr int kPSlices = 64;        // slices per block, at most (2048 rows)
 constexpr unsigned kPollLimit = 1u << 22;  // polls of one barrier before it gives up (seconds)
@@ -84,7 +92,7 @@ struct PArgs {
   double2* rq;            // grid form: r and q of every row
   double* ay;
   double* yz;             // y, then z (and x for the true residual)
-  PSlot* slots;           // grid form: [2 parities][kPMaxBlocks]
+  PSlot* slots;           // grid form: [kPSlotSets][kPMaxBlocks]
   SolveOut* out;
   double tol;
   int tol_mode, maxiter, verify;
@@ -417,11 +425,11 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
   unsigned ep = 0;
   double tot[2] = {0.0, 0.0};
   // near (grid form, nd = 0): wait only for the blocks whose rows this one
-  // gathers.  Nothing they write is overwritten, and no slot reused, before the
-  // next barrier of all blocks: two near ones never follow each other.
+  // gathers.  Nothing they write is overwritten before the next barrier of all
+  // blocks, and no slot before such a barrier has passed (kPSlotSets): two near
+  // ones never follow each other.
   auto sync = [&](int nd, double v0, double v1, bool near = false) -> bool {
     ++ep;
-    const unsigned par = ep & 1u;
     if (nd > 0) {
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) {
@@ -434,6 +442,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       }
     }
     if constexpr (CL) {
+      const unsigned par = ep & 1u;
       if (nd > 0) {
         __syncthreads();
         if (wid == 0) {
@@ -463,6 +472,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
       // share lines take 4.5 us a barrier on one B200, 2.2 us on lines of their
       // own; fences and the two trips through L2 are the rest).
       __syncthreads();
+      PSlot* const set = a.slots + (ep % kPSlotSets) * kPMaxBlocks;
       const int nsum = max(nd, 1);
       bool lost = false;
       if (wid == 0) {
@@ -483,7 +493,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
           const unsigned long long u = nd > 0 ? (unsigned long long)__double_as_longlong(s0) : 0ull;
           const unsigned long long lo = (u & 0xffffffffull) | ((unsigned long long)ep << 32);
           const unsigned long long hi = (u >> 32) | ((unsigned long long)ep << 32);
-          PSlot* dst = a.slots + par * kPMaxBlocks + bid;
+          PSlot* dst = set + bid;
           asm volatile("fence.acq_rel.gpu;" ::: "memory");
           asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" : : "l"(&dst->v[lane]), "l"(lo), "l"(hi)
                        : "memory");
@@ -501,7 +511,7 @@ __global__ void __launch_bounds__(PT, 1) k_bi_persist(PArgs a) {
 #pragma unroll
           for (int m = 0; m < kPPoll; ++m) {
             if (got >> m & 1u) continue;
-            const PSlot* src = a.slots + par * kPMaxBlocks + lane + 32 * m;
+            const PSlot* src = set + lane + 32 * m;
             bool seen = true;
 #pragma unroll
             for (int d = 0; d < 2; ++d) {
@@ -856,7 +866,7 @@ int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* m
   if (bytes(form) > c->smem_optin) return DCU_OK;
   const size_t smem = bytes(form) - kPStatic;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  const size_t nslot = sh.cluster ? 0 : sizeof(PSlot) * 2 * kPMaxBlocks;
+  const size_t nslot = sh.cluster ? 0 : sizeof(PSlot) * kPSlotSets * kPMaxBlocks;
   const size_t vec = al(sizeof(double) * (size_t)plan.n);
   DCU_TRY(ensure(c, B_PERSIST, al(sizeof(SolveOut)) + nslot + (sh.cluster ? 0 : 4 * vec)));
   char* base = bp<char>(c, B_PERSIST);
