@@ -602,6 +602,7 @@ struct BCArgs {
   double tol;
   int tol_mode, maxiter;
   int cap;                  // doubles of dynamic shared memory
+  int* last;                // the batch's iteration counter: the latest that any system reached
   int* iters;
   int* status;
 };
@@ -1050,6 +1051,8 @@ __global__ void __launch_bounds__(BC_THREADS, 1) k_batch_cluster(BCArgs a) {
     if (rank == 0 && tid < R) {
       a.iters[(size_t)sys * R + tid] = conv[tid];
       a.status[(size_t)sys * R + tid] = stat[tid] < 0 ? DCU_SOLVE_MAXITER : stat[tid];
+      // (kb_step's counter: it stays on the iteration in which the last pair stopped)
+      if (tid == 0) atomicMax(a.last, live == 0 ? max(1, it - 1) : it);
     }
     __syncthreads();
   }
@@ -1145,7 +1148,7 @@ int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector
   }
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
   const size_t vec = al(sizeof(double) * (size_t)n * R), pairs = (size_t)nsys * R;
-  const size_t heads = al(sizeof(int) * 3 * cls.size());
+  const size_t heads = al(sizeof(int) * (3 * cls.size() + 1));
   DCU_TRY(ensure(c, B_VEC, 7 * vec + heads + al(sizeof(int) * nsys) + 2 * al(sizeof(int) * pairs)));
   char* p = bp<char>(c, B_VEC);
   BCArgs a{};
@@ -1161,6 +1164,7 @@ int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector
   double** vecs[7] = {&a.r, &a.q, &a.y, &a.ay, &a.z, &a.rs, &a.az};
   for (int i = 0; i < 7; ++i) *vecs[i] = reinterpret_cast<double*>(p + i * vec);
   int* head = reinterpret_cast<int*>(p + 7 * vec);
+  a.last = head + 3 * cls.size();
   int* ord = reinterpret_cast<int*>(p + 7 * vec + heads);
   a.iters = reinterpret_cast<int*>(p + 7 * vec + heads + al(sizeof(int) * nsys));
   a.status = reinterpret_cast<int*>(p + 7 * vec + heads + al(sizeof(int) * nsys) + al(sizeof(int) * pairs));
@@ -1190,15 +1194,14 @@ int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector
   DCU_CUDA(c, cudaEventRecord(c->ev[1], c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(iters_h, a.iters, sizeof(int) * pairs, cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(status_h, a.status, sizeof(int) * pairs, cudaMemcpyDeviceToHost, c->stream));
+  int* last = static_cast<int*>(c->pinned);
+  DCU_CUDA(c, cudaMemcpyAsync(last, a.last, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaStreamSynchronize(c->stream));
   *ran = true;
   if (info) {
-    info->iters = 1;
+    info->iters = *last;
     info->status = DCU_SOLVE_CONVERGED;
-    for (size_t i = 0; i < pairs; ++i) {
-      info->iters = std::max(info->iters, iters_h[i]);
-      info->status = std::max(info->status, status_h[i]);
-    }
+    for (size_t i = 0; i < pairs; ++i) info->status = std::max(info->status, status_h[i]);
     info->replacements = 0;
     info->res = info->true_res = info->bnorm = 0.0;
     info->a_fp32 = 0;

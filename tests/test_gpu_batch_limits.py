@@ -3,6 +3,7 @@ batch's iteration counter when a pair breaks down inside an iteration."""
 import numpy as np
 import pytest
 
+from dcu_b200 import native as N
 from dcu_b200 import workloads as W
 from dcu_b200.api import DcuError
 
@@ -25,3 +26,16 @@ def test_a_batch_without_rows_is_refused(ctx, nsys, nrhs):
     A = W.convdiff2d(4, 10.0)
     with pytest.raises(DcuError, match="empty batch"):
         _solve(ctx, A, [0] * (nsys + 1), np.ones((A.n, nrhs)))
+
+
+def test_counter_of_a_breakdown_inside_an_iteration(ctx):
+    """A cyclic shift (M = 0 there) beside a diagonal: exact arithmetic, r = (b1, 0) after the first
+    iteration, y = M p = 0 in the second, (r*, A y) = 0.  The pair stopped with one finished iteration, the
+    batch in its second."""
+    n = 6
+    cols = [[1], [2], [0], [3], [4], [5]]
+    A = W.CSC(n, np.arange(n + 1, dtype=np.int32), np.concatenate(cols).astype(np.int32), np.ones(n))
+    # |b1|^2 = |b2|^2: alpha = 2
+    X, it, st, _, si = _solve(ctx, A, [0, n], np.ones((n, 1)), tol=1e-10)
+    assert st[0, 0] == N.SOLVE_BREAKDOWN and it[0, 0] == 1 and si.iters == 2
+    assert np.array_equal(X[:, 0], [0.0, 0.0, 0.0, 1.0, 1.0, 1.0])
