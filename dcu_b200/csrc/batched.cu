@@ -13,6 +13,8 @@
 // system to finish sums that system's partials in tile order (deterministic)
 // and updates the system's scalars.
 #include <algorithm>
+#include <climits>
+#include <cmath>
 
 #include "internal.cuh"
 
@@ -1071,27 +1073,66 @@ __global__ void kb_check_blocks(const int* __restrict__ ptr, const int* __restri
   }
 }
 
-// Whether a batch goes to the clusters.  In units of one row x right-hand side
-// of a 16-CTA cluster's iteration (about 0.5 ns; seven such clusters run at
-// once): a cluster's iteration costs its rows and a fixed 20000 (five
-// barriers), the tile kernels' the whole batch's rows at a rate that grows with
-// the right-hand sides (they are bound by HBM, the clusters by L1) and a fixed
-// 48000 (six launches).  Measured on one B200, tile kernels -> clusters: 128 systems
-// of 300-4000 rows x 8 6.9 -> 4.3 ms, 256 of 300-50000 x 4 53.9 -> 44.1, x 2 37.1 ->
-// 24.5, x 1 32.6 -> 19.4, 16 small ones 2.6 -> 1.1; 512 of 1000-50000 x 8 equal, 8 of
-// 300-50000 x 4 9.0 -> 9.7 (too few large systems to fill the clusters).
+// CTAs of a system's cluster: two passes of rows each, up to 16.
+template <int R>
+int batch_ctas(int rows) {
+  int k = 1;
+  while (k < BC_MAXC && rows > 2 * BCEntries<R>::ROWS * k) k <<= 1;
+  return k;
+}
+
+// Whether a batch goes to the clusters: two estimates of the time of one
+// iteration of all its systems, in us on one B200, a system of n rows counted
+// sqrt(n / largest) times (the iterations of a stencil grow with its width).
+//   clusters  a system's iteration takes 3.7 us and 5.6 to 7.2 us for every pass
+//             of its CTAs' rows (a fifth more at 8 right-hand sides once r* of
+//             the rows no longer fits shared memory); 148, 74, 33, 15 and 7
+//             clusters of 1, 2, 4, 8 and 16 CTAs run at once, one after
+//             another.  At least the longest system, and whole rounds of every
+//             class.
+//   tiles     six launches, the tiles, their rows, and the last tile's sum over
+//             its system's tiles.
+// The constants are fitted to batches of 1 to 8192 equal systems of 16 to 90000
+// rows.  The clusters may be estimated up to 1.2 times as long: a cluster
+// costs a system's own iterations, the tiles' launches go on until the last
+// system stops, and equal sizes converge apart too; less with more right-hand
+// sides, where rows outweigh launches.  Of 156 batches with random sizes and
+// coefficients the rule is never over 1.04 times the tiles' time, nor over 1.18
+// times the faster one's.  Solve times, tiles and clusters, ms: 4096 systems of 64
+// rows x 1 2.3 and 3.1; 2048 of 100 to 300 x 4 3.7 and 3.1; 1000 of 300 to 1000
+// x 1 3.0 and 2.0; 300 of 300 to 4000 x 8 7.6 and 8.8, x 1 2.8 and 1.8; 64 of 20000
+// to 50000 x 1 30 and 22, x 8 92 and 120.
 template <int R>
 bool cluster_batch(const std::vector<int>& so, int nsys) {
-  double sum = 0.0, most = 0.0;
-  int rows = 0;
+  constexpr double pass_us = R == 1 ? 5.6 : R == 2 ? 7.2 : R == 4 ? 6.9 : 7.0;
+  constexpr double row_us = R == 1 ? 25e-6 : R == 2 ? 28e-6 : R == 4 ? 33e-6 : 34e-6;
+  constexpr double slack = R <= 2 ? 1.2 : 1.15;
+  constexpr int own = R == 8 ? (int)((64 * 1024 - bc_entry_bytes<R>()) / (sizeof(double) * R)) : INT_MAX;
+  constexpr int resident[5] = {148, 74, 33, 15, 7};
+  int tall = 0;
+  for (int s = 0; s < nsys; ++s) tall = std::max(tall, so[s + 1] - so[s]);
+  if (tall > BC_MAXC * (32 * (BC_SLICES - 2) - 8)) return false;  // slices of a CTA
+  double tiles = 23.5 + 2.0 * R * std::min(1.0, tall / (double)BT) + 0.1 * ((tall + BT - 1) / BT);
+  double class_us[5] = {}, most = 0.0, all = 0.0;
+  int class_n[5] = {};
   for (int s = 0; s < nsys; ++s) {
     const int n = so[s + 1] - so[s];
-    rows = std::max(rows, n);
-    sum += (double)n * R;
-    most = std::max(most, 20000.0 + (R <= 2 ? 0.6 : 1.0) * n * R);
+    if (n <= 0) continue;
+    const int k = batch_ctas<R>(n), rpc = (n + k - 1) / k;
+    const int passes = (rpc + BCEntries<R>::ROWS - 1) / BCEntries<R>::ROWS;
+    const int c = k == 1 ? 0 : k == 2 ? 1 : k == 4 ? 2 : k == 8 ? 3 : 4;
+    const double w = std::sqrt((double)n / tall), us = w * (3.7 + (rpc > own ? 1.2 : 1.0) * pass_us * passes);
+    ++class_n[c];
+    class_us[c] += us;
+    most = std::max(most, us);
+    tiles += w * ((n + BT - 1) / BT * (0.018 + 0.002 * R) + n * R * row_us);
   }
-  if (rows > BC_MAXC * (32 * (BC_SLICES - 2) - 8)) return false;  // slices of a CTA
-  return std::max(sum / 7.0, most) < 48000.0 + sum * (R == 8 ? 0.14 : R == 4 ? 0.17 : 0.3);
+  for (int c = 0; c < 5; ++c) {
+    if (class_n[c] == 0) continue;
+    all += class_us[c] / resident[c];
+    most = std::max(most, (class_n[c] + resident[c] - 1) / resident[c] * class_us[c] / class_n[c]);
+  }
+  return std::max(all, most) < slack * tiles;
 }
 
 // The systems of a batch through k_batch_cluster: classes by size, the larger
@@ -1112,19 +1153,12 @@ int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector
   std::vector<int> order(nsys);
   for (int s = 0; s < nsys; ++s) order[s] = s;
   std::stable_sort(order.begin(), order.end(), [&](int p, int q) { return so[p + 1] - so[p] > so[q + 1] - so[q]; });
-  // CTAs per system: two passes of rows each, up to 16
-  const int unit = BCEntries<R>::ROWS;
-  auto ctas = [&](int rows) {
-    int k = 1;
-    while (k < BC_MAXC && rows > 2 * unit * k) k <<= 1;
-    return k;
-  };
   struct Class {
     int cta, first, count, grid;
   };
   std::vector<Class> cls;
   for (int i = 0; i < nsys; ++i) {
-    const int k = ctas(so[order[i] + 1] - so[order[i]]);
+    const int k = batch_ctas<R>(so[order[i] + 1] - so[order[i]]);
     if (cls.empty() || cls.back().cta != k) cls.push_back({k, i, 0, 0});
     ++cls.back().count;
   }

@@ -39,3 +39,21 @@ def test_counter_of_a_breakdown_inside_an_iteration(ctx):
     X, it, st, _, si = _solve(ctx, A, [0, n], np.ones((n, 1)), tol=1e-10)
     assert st[0, 0] == N.SOLVE_BREAKDOWN and it[0, 0] == 1 and si.iters == 2
     assert np.array_equal(X[:, 0], [0.0, 0.0, 0.0, 1.0, 1.0, 1.0])
+
+
+@pytest.mark.parametrize("count,rows,nrhs,tiles", [(4096, 16, 1, True), (100, 16, 1, False), (3000, 64, 2, True), (140, 64, 8, False)])
+def test_many_small_systems_go_to_the_tiles(ctx, count, rows, nrhs, tiles):
+    """Clusters pay a fixed time a system and iteration: hundreds at once, not thousands one after another."""
+    P = W.convdiff2d(int(rows ** 0.5), 10.0)
+    k = np.arange(count)[:, None]
+    ptr = np.concatenate([[0], (P.ptr[None, 1:] + P.nnz * k).ravel()]).astype(np.int32)
+    A = W.CSC(P.n * count, ptr, (P.idx[None, :] + P.n * k).ravel().astype(np.int32), np.tile(P.val, count))
+    Xt = np.random.default_rng(1).standard_normal((A.n, nrhs))
+    B = np.stack([A.matvec(Xt[:, q]) for q in range(nrhs)], 1)
+    before = ctx.launches
+    X, it, st, _, si = _solve(ctx, A, np.arange(count + 1) * P.n, B, tol=1e-10)
+    launches = ctx.launches - before
+    assert (st == N.SOLVE_CONVERGED).all()
+    assert np.linalg.norm(X - Xt) <= 1e-8 * np.linalg.norm(Xt)
+    # the tiles take five launches an iteration and more, the clusters one a size
+    assert (launches > 5 * it.max()) == tiles
