@@ -262,7 +262,8 @@ int validate_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, bool un
 // CSR of a CSC matrix (with val and rval its values too); the stream is idle on return.
 int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rptr, int* rcol, int* rperm,
                  const double* val, double* rval);
-int csr_values(Ctx* c, int nnz, const int* rperm, const double* val, double* rval);
+// (skip: device flag, the values are left alone when it is set)
+int csr_values(Ctx* c, int nnz, const int* rperm, const double* val, double* rval, const int* skip = nullptr);
 int sell_plan(Ctx* c, int n, int nnz, const int* ptr, const int* idx, SellPlan* plan);
 // SELL-32 layout of the operator whose CSR is (rptr, rcol, rperm).  With
 // `check` (a device int), its value is read back with the layout's last

@@ -300,12 +300,11 @@ __global__ void __launch_bounds__(512) k_row_sort_long(const int* __restrict__ r
   }
 }
 
+// (nothing when *skip, where given, is set: the map does not stand)
 __global__ void k_gather_f64(const int* __restrict__ perm, const double* __restrict__ src, int nnz,
-                             double* __restrict__ dst) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) {
-    const int p = perm[e];
-    if (p >= 0) dst[e] = src[p];
-  }
+                             double* __restrict__ dst, const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) dst[e] = src[perm[e]];
 }
 
 // SELL: slice widths (max row length of each 32-row slice), one warp per slice.
@@ -701,8 +700,8 @@ int csr_from_csc(Ctx* c, int n, int nnz, const int* ptr, const int* idx, int* rp
   if (n > 0 && nnz > 0) {
     int* flag = nullptr;
     DCU_TRY(csr_try_symmetric(c, n, ptr, idx, rptr, rcol, rperm, &flag, true));
-    // the values without waiting for the verdict (a slot without a partner is -1)
-    if (val && rval) DCU_TRY(csr_values(c, nnz, rperm, val, rval));
+    // the values without waiting for the verdict, which the gather reads itself
+    if (val && rval) DCU_TRY(csr_values(c, nnz, rperm, val, rval, flag));
     DCU_CUDA(c, cudaMemcpyAsync(c->pinned, flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     DCU_CUDA(c, cudaStreamSynchronize(c->stream));
     if (*(int*)c->pinned == 0) return DCU_OK;
@@ -929,9 +928,9 @@ int sell_gather_m8_bf16(Ctx* c, const SellPlan& p, const double* src, __nv_bfloa
 }
 
 // CSR with values, for the C ABI (dcu_csc_to_csr_d).
-int csr_values(Ctx* c, int nnz, const int* rperm, const double* val, double* rval) {
+int csr_values(Ctx* c, int nnz, const int* rperm, const double* val, double* rval, const int* skip) {
   if (nnz <= 0 || !rval) return DCU_OK;
-  k_gather_f64<<<waves_grid(c, nnz, 256, 8), 256, 0, c->stream>>>(rperm, val, nnz, rval);
+  k_gather_f64<<<waves_grid(c, nnz, 256, 8), 256, 0, c->stream>>>(rperm, val, nnz, rval, skip);
   DCU_LAUNCHED(c, "k_gather_f64");
   return DCU_OK;
 }
@@ -1091,7 +1090,7 @@ extern "C" int dcu_csc_to_csr_noalloc_d(int n, int nnz, const int* ptr, const in
   k_row_sort_long_smem<<<148, 512, smem, st>>>(rptr, longrows, longcount, ridx, perm, flags);
   NOALLOC_CHECK(cudaGetLastError());
   if (val && rval && nnz > 0) {
-    k_gather_f64<<<grid_z, 256, 0, st>>>(perm, val, nnz, rval);
+    k_gather_f64<<<grid_z, 256, 0, st>>>(perm, val, nnz, rval, nullptr);
     NOALLOC_CHECK(cudaGetLastError());
   }
   NOALLOC_CHECK(cudaMemcpyAsync(host_flags, flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
