@@ -2511,9 +2511,15 @@ int build_finish(Ctx* c, int n, const int* ptr, const int* idx, const double* va
     la.area_per_block = area;
     memcpy(&la.area_sum, reinterpret_cast<long long*>(st) + ST_AREASUM64, sizeof la.area_sum);
     J->finish_launched = true;
+    // In FP64 as the hand-offs above while that costs nothing: at most a column an
+    // SM (hubs: the FP64 panels take 0.7 to 0.8 of the FP32 steps' solve), or few
+    // entries in all.  Whole calls, FP32 / FP64: 2400 columns of 3 M entries 2.9 /
+    // 2.9 ms, 12000 of 30 M 3.2 / 3.3; 19000 of 40 M 3.3 / 3.5, 20000 of 77 M 4.5 /
+    // 4.9, 20000 of 547 M 15.2 / 22.3 (their blocks leave a CTA's shared memory).
+    constexpr long long kLarge64 = 1ll << 25;
     const bool v64 = J->opt.precision == DCU_PREC_M_FP32 || J->opt.precision == DCU_PREC_M_BF16;
-    if (std::is_same<T, float>::value && v64 && J->thread_path)
-      DCU_TRY((run_large<double, MODE_BUILD>(c, la, nbig, cta_max_area)));  // (as the hand-offs above)
+    if (std::is_same<T, float>::value && v64 && J->thread_path && (nbig <= c->sms || la.area_sum <= kLarge64))
+      DCU_TRY((run_large<double, MODE_BUILD>(c, la, nbig, cta_max_area)));
     else
       DCU_TRY((run_large<T, MODE_BUILD>(c, la, nbig, cta_max_area)));
     DCU_TRY(read_stats(c, st));
