@@ -208,14 +208,16 @@ struct SellPlan {
   const int* rptr = nullptr;  // CSR row pointers of the laid-out operator (row lengths)
   const int* wide = nullptr;  // the slices flagged wide (device)
   int nwide = 0;
-  // one-launch solver (persist.cu): most slots and most segments of long rows
-  // any of its blocks holds; 0 slots when it does not take an operator of this size
-  int max_block_slots = 0, max_block_long = 0;
+  // one-launch solver (persist.cu), its first shape for this size and the second:
+  // most slots and most segments of long rows any of its blocks holds; 0 slots
+  // when there is no such shape
+  int max_block_slots[2] = {0, 0}, max_block_long[2] = {0, 0};
   long long uniform_slots = 0;  // slots in offset-uniform slices
 };
 
 // How the one-launch solver splits an operator of n rows: `blocks` blocks
-// (0: too large for it) of `spb` 32-row slices each.
+// (0: too large for it) of `spb` 32-row slices each.  An operator for one
+// cluster has a second shape, the grid form (for scattered columns).
 struct PersistShape {
   bool cluster = false;
   int spb = 0, blocks = 0;
@@ -240,7 +242,7 @@ __device__ __forceinline__ bool slice_split(int w, int len) {
   return w > kPersistLong && (nlong <= kWideRows || total < 8 * w);
 }
 #endif
-PersistShape persist_shape(const Ctx* c, int n);
+PersistShape persist_shape(const Ctx* c, int n, bool second = false);
 
 // What the one-launch solver writes at its end.
 struct SolveOut {

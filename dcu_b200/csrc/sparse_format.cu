@@ -346,7 +346,8 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
                               int* __restrict__ sidx, int* __restrict__ sperm, int* __restrict__ maxdelta,
                               int16_t* __restrict__ del, int* __restrict__ kd, int* __restrict__ su,
                               unsigned long long* __restrict__ uslots, int* __restrict__ wide, int allow_wide,
-                              int* __restrict__ kd8, int16_t* __restrict__ kd8h, int* __restrict__ cost, int spb) {
+                              int* __restrict__ kd8, int16_t* __restrict__ kd8h, int* __restrict__ cost, int spb,
+                              int* __restrict__ cost2, int spb2) {
   __shared__ unsigned long long blk_uslots;
   if (threadIdx.x == 0) blk_uslots = 0ull;
   __syncthreads();
@@ -424,8 +425,9 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       kd8[(long long)s * kNarrow + lane] = d;
       kd8h[(long long)s * kNarrow + lane] = (int16_t)d;  // read only when every |d| < 32768
     }
-    // the slice's share of a block of the one-launch solver (persist.cu, which
-    // makes the same split): slots kept, entries and segments of the long rows
+    // the slice's share of a block of the one-launch solver, in its first shape
+    // and the second (persist.cu, which makes the same split): slots kept,
+    // entries and segments of the long rows
     if (spb > 0) {
       const bool split = sparse;
       const int ws = __reduce_max_sync(0xffffffffu, !split ? w : (len <= kPersistLong ? len : 0));
@@ -434,6 +436,10 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       if (lane == 0) {
         atomicAdd(&cost[2 * (s / spb)], 32 * ws + le);
         if (nl) atomicAdd(&cost[2 * (s / spb) + 1], nl);
+        if (spb2 > 0) {
+          atomicAdd(&cost2[2 * (s / spb2)], 32 * ws + le);
+          if (nl) atomicAdd(&cost2[2 * (s / spb2) + 1], nl);
+        }
       }
     }
     if (lane == 0) {
@@ -766,9 +772,10 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   int* kd = su + nslices;
   // slots, uniform slots; then per block of the one-launch solver its slots and
   // segments of long rows
-  const PersistShape ps = persist_shape(c, n);
+  const PersistShape ps[2] = {persist_shape(c, n), persist_shape(c, n, true)};
+  const int nblocks = ps[0].blocks + ps[1].blocks;  // (16 + 32 at most where there is a second shape)
   unsigned long long hst[2 + kPersistBlocks] = {(unsigned long long)slots};
-  const size_t nst = sizeof(unsigned long long) * (2 + (size_t)ps.blocks);
+  const size_t nst = sizeof(unsigned long long) * (2 + (size_t)nblocks);
   DCU_TRY(ensure(c, B_PLANSTAT, sizeof(hst)));
   unsigned long long* pst = bp<unsigned long long>(c, B_PLANSTAT);
   int* cost = reinterpret_cast<int*>(pst + 2);
@@ -781,12 +788,12 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   DCU_CUDA(c, cudaMemsetAsync(wide, 0, sizeof(int), c->stream));
   k_sell_layout<<<waves_grid(c, (long long)nslices * 32, 256, 8), 256, 0, c->stream>>>(
       rptr, rcol, rperm, n, nslices, off, sidx, sperm, maxdelta, del, kd, su, pst + 1, wide, c->wide_prepass ? 1 : 0,
-      kd8, kd8h, cost, ps.blocks > 0 ? ps.spb : 0);
+      kd8, kd8h, cost, ps[0].blocks > 0 ? ps[0].spb : 0, cost + 2 * ps[0].blocks, ps[1].blocks > 0 ? ps[1].spb : 0);
   DCU_LAUNCHED(c, "k_sell_layout");
   // [0] wide slices, [1] largest delta, [2] check, then uniform slots and the blocks' costs
   int* hcost = reinterpret_cast<int*>(c->pinned) + 4;
   static_assert(sizeof(int) * (6 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
-  DCU_CUDA(c, cudaMemcpyAsync(hcost, pst + 1, sizeof(unsigned long long) * (1 + (size_t)ps.blocks),
+  DCU_CUDA(c, cudaMemcpyAsync(hcost, pst + 1, sizeof(unsigned long long) * (1 + (size_t)nblocks),
                               cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(c->pinned, wide, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(reinterpret_cast<int*>(c->pinned) + 1, maxdelta, sizeof(int), cudaMemcpyDeviceToHost,
@@ -799,10 +806,12 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   plan->nwide = *reinterpret_cast<int*>(c->pinned);
   std::memcpy(&plan->uniform_slots, hcost, sizeof(long long));
   hcost += 2;
-  plan->max_block_slots = plan->max_block_long = 0;
-  for (int g = 0; g < ps.blocks; ++g) {
-    plan->max_block_slots = std::max(plan->max_block_slots, hcost[2 * g]);
-    plan->max_block_long = std::max(plan->max_block_long, hcost[2 * g + 1]);
+  for (int k = 0; k < 2; ++k) {
+    plan->max_block_slots[k] = plan->max_block_long[k] = 0;
+    for (int g = 0; g < ps[k].blocks; ++g, hcost += 2) {
+      plan->max_block_slots[k] = std::max(plan->max_block_slots[k], hcost[0]);
+      plan->max_block_long[k] = std::max(plan->max_block_long[k], hcost[1]);
+    }
   }
   plan->delta16 = reinterpret_cast<int*>(c->pinned)[1] < 32768;
   plan->del = plan->delta16 ? del : nullptr;
