@@ -359,7 +359,10 @@ int autotune(Ctx* c, int n, int nnz, const int* ptr, const int* idx, const doubl
   }
   const int iters = si.iters > 0 ? si.iters : 1;
   t->k1_split = cands[pick].k1_split;
-  if (c->profile_one_launch && c->profile_k1_free) t->k1_split = c->profile_default_split;
+  // Nothing was measured for an operator that solves in one launch: its form's
+  // default stands, by its value where that is the same at every size; plain
+  // FP64's depends on the entries, and a larger operator must still find its own.
+  if (c->profile_one_launch && c->profile_k1_free && p != DCU_PREC_FP64) t->k1_split = c->profile_default_split;
   t->grid_p = cands[pick].grid_p;
   t->grid_y = cands[pick].grid_y;
   t->grid_py = cands[pick].grid_py;
