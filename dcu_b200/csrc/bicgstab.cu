@@ -967,8 +967,11 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
         info->a_fp32 = o.a32;
         cudaEventElapsedTime(&info->ms, c->ev[0], c->ev[1]);
       }
-      // the profiling launches start from clean scalars and counters (not waited for)
+      // the profiling launches start from clean scalars and counters, and read A
+      // as the solve did: its FP64 array may be absent (not waited for)
       DCU_CUDA(c, cudaMemsetAsync(a.S, 0, sizeof(Scal), c->stream));
+      DCU_CUDA(c, cudaMemcpyAsync(&a.S->a32, &bp<SolveOut>(c, B_PERSIST)->a32, sizeof(int), cudaMemcpyDeviceToDevice,
+                                  c->stream));
       return DCU_OK;
     }
   }
