@@ -502,6 +502,7 @@ struct GroupArgs {
   int* wide_list;  // GroupC's columns
   const int* in;   // this kernel's columns (null: the range) ...
   int in_count;    // ... and the stats[] entry that counts them
+  int limit;       // a column with more rows than this goes to the CTA kernel (INT_MAX: none by its rows)
 };
 
 template <typename T, typename S>
@@ -848,8 +849,8 @@ __device__ __forceinline__ int rows_stage_lists(GroupSmem<T, S>& gs, int k, cons
   return m;
 }
 
+// (5 blocks an SM for the first two sizes; held to 6 they spill: 128^3 build 1.54 -> 1.58 ms)
 template <typename T, typename S>
-// (6 blocks an SM for the first two sizes without spilling in the steps)
 __global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(GroupArgs ga) {
   extern __shared__ __align__(16) unsigned char rows_raw[];
   const SmallArgs& a = ga.a;
@@ -861,9 +862,12 @@ __global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(Grou
   const int nwarps = (gridDim.x * GR_BLOCK) >> 5;
   int my_max_ni = 0, my_max_nj = 0, my_cols = 0, my_sing = 0;
 
-  // the next size for a column this one does not take (lane 0 of its group)
-  auto pass_on = [&](int k, int nj, long long cand) {
-    if (ga.mid_list && S::NJ < GroupB::NJ && nj <= GroupB::NJ && cand <= GroupB::CMAX)
+  // the next size for a column this one does not take (lane 0 of its group);
+  // m = INT_MAX where its rows are not known
+  auto pass_on = [&](int k, int nj, long long cand, int m) {
+    if (m > ga.limit)
+      queue_big(a, k, nj, cand * (nj + 1));
+    else if (ga.mid_list && S::NJ < GroupB::NJ && nj <= GroupB::NJ && cand <= GroupB::CMAX)
       ga.mid_list[atomicAdd(&a.stats[ST_MID_COUNT], 1)] = k;
     else if (ga.mid_list && S::NJ < GroupC::NJ && nj <= GroupC::NJ && cand <= GroupC::CMAX)
       ga.wide_list[atomicAdd(&a.stats[ST_WIDE_COUNT], 1)] = k;
@@ -892,7 +896,7 @@ __global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(Grou
         }
       cand = group_sum<G>(cand);
       if (nj > S::NJ) {
-        if (lane == 0) pass_on(k, nj, cand);
+        if (lane == 0) pass_on(k, nj, cand, INT_MAX);
         nj = 0;
       }
     }
@@ -957,7 +961,7 @@ __global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(Grou
         c2 += __shfl_sync(0xffffffffu, inc, G - 1, G);
       }
       if (c2 > S::CMAX) {
-        if (lane == 0) pass_on(k, nj, c2);
+        if (lane == 0) pass_on(k, nj, c2, INT_MAX);
         nj = 0;
         c2 = 0;
       }
@@ -969,7 +973,7 @@ __global__ void __launch_bounds__(GR_BLOCK, S::G == 16 ? 4 : 5) k_spai_rows(Grou
     }
     if (nj > 0) {
       if (m > max_ni) {
-        if (lane == 0) pass_on(k, nj, c2);
+        if (lane == 0) pass_on(k, nj, c2, m);
         nj = 0;
         m = 0;
       } else {
@@ -2174,14 +2178,16 @@ int launch_rows(Ctx* c, GroupArgs ga) {
 }
 
 // First size: the range, or the columns the thread kernel handed over.  With
-// a tuned |I| limit the columns above it go to the CTA kernel.
+// a tuned |I| limit the columns above it go to the CTA kernel, and so do those
+// that are too wide for the first size.
 template <typename T>
 int run_rows(Ctx* c, const SmallArgs& sa) {
   GroupArgs ga{};
   ga.a = sa;
   ga.in = sa.list;
   ga.in_count = ST_FB_COUNT;
-  if (sa.max_ni >= SG_MMAX) {
+  ga.limit = sa.max_ni >= SG_MMAX ? INT_MAX : sa.max_ni;
+  if (sa.max_ni > GroupA::RMAX) {
     const size_t n = (size_t)std::max(1, sa.col_end - sa.col_start);
     DCU_TRY(ensure(c, B_MIDLIST, sizeof(int) * 2 * n));
     ga.mid_list = bp<int>(c, B_MIDLIST);
@@ -2197,7 +2203,7 @@ int run_rows_rest(Ctx* c, const SmallArgs& sa, int mid) {
   ga.a = sa;
   ga.mid_list = bp<int>(c, B_MIDLIST);
   ga.wide_list = ga.mid_list + std::max(1, sa.col_end - sa.col_start);
-  ga.a.max_ni = INT_MAX;
+  ga.a.max_ni = ga.limit = INT_MAX;
   if (mid > 0) {
     ga.in = ga.mid_list;
     ga.in_count = ST_MID_COUNT;
