@@ -65,15 +65,17 @@ bool a32_copy(const Ctx* c, const dcu::SellPlan& plan, int precision) {
   return c->exact_a32 && (precision != DCU_PREC_FP64 || plan.slots >= kA32Slots);
 }
 
-// A's values in SELL order: FP64, and with `copy` the FP32 copy with its
-// exactness flag.  With the copy exact and no wide slice the FP64 array is not
+// A's values in SELL order for a solve in form `precision`: FP64, and with
+// `copy` the FP32 copy with its exactness flag.  With the copy exact and no wide slice the FP64 array is not
 // written: only a reader of the flag may ask for it (the solvers of single
 // systems; the batched kernels read FP64 values).
-int gather_a(Ctx* c, const dcu::SellPlan& plan, const double* val, bool copy, dcu::SellA* a) {
+int gather_a(Ctx* c, const dcu::SellPlan& plan, const double* val, int precision, bool copy, dcu::SellA* a) {
   const size_t slots = (size_t)(plan.slots > 0 ? plan.slots : 1);
   DCU_TRY(dcu::ensure(c, dcu::B_SELL_AVAL, sizeof(double) * slots));
   *a = dcu::SellA{};
   a->v64 = dcu::bp<double>(c, dcu::B_SELL_AVAL);
+  // the plain form solves without the copy where there is no room for it
+  if (copy && precision == DCU_PREC_FP64) copy = dcu::ensure_optional(c, dcu::B_SELL_AVAL32, sizeof(float) * slots);
   if (!copy)
     return dcu::sell_gather_f64(c, plan, val, dcu::bp<double>(c, dcu::B_SELL_AVAL));
   DCU_TRY(dcu::ensure(c, dcu::B_SELL_AVAL32, sizeof(float) * slots));
@@ -113,7 +115,7 @@ int gather_m(Ctx* c, const dcu::SellPlan& pl, const double* mval, int precision,
 // A's values and M's (by form) in SELL order.
 int gather_values(Ctx* c, const dcu::SellPlan& plan, const double* val, const double* mval, int precision,
                   dcu::SellA* asell, const void** msell, const void** msell8) {
-  DCU_TRY(gather_a(c, plan, val, a32_copy(c, plan, precision), asell));
+  DCU_TRY(gather_a(c, plan, val, precision, a32_copy(c, plan, precision), asell));
   return gather_m(c, plan, mval, precision, msell, msell8);
 }
 
@@ -167,7 +169,7 @@ int solve_pipeline(Ctx* c, int n, int nnz, const int* ptr, const int* idx, const
     DCU_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev[6], 0));
     DCU_TRY(dcu::sell_plan(c, n, nnz, ptr, idx, &plan));
     if (val_ready) DCU_CUDA(c, cudaStreamWaitEvent(c->stream, val_ready, 0));
-    DCU_TRY(gather_a(c, plan, val, a32_copy(c, plan, o.precision), &asell));
+    DCU_TRY(gather_a(c, plan, val, o.precision, a32_copy(c, plan, o.precision), &asell));
     DCU_CUDA(c, cudaEventRecord(c->ev[7], c->stream));
   }
   DCU_TRY(dcu::spai_build_finish(c, &job, &bl));
@@ -772,7 +774,7 @@ int dcu_batch_solve_d(dcu_spai_ctx* c, int nsys, const int* sys_off, int n, int 
     dcu::SellA asell;
     const void *msell = nullptr, *msell8 = nullptr;
     DCU_TRY(dcu::sell_plan(c, n, nnz, ptr, idx, &plan));
-    DCU_TRY(gather_a(c, plan, val, /*copy=*/false, &asell));
+    DCU_TRY(gather_a(c, plan, val, DCU_PREC_FP64, /*copy=*/false, &asell));
     DCU_TRY(gather_m(c, plan, m, DCU_PREC_FP64, &msell, &msell8));
     return dcu::batch_solve(c, nsys, sys_off, plan, asell.v64, (const double*)msell,
                             nrhs, B, X, &o, iters, status, sinfo);

@@ -156,6 +156,9 @@ int cuda_fail(Ctx* c, cudaError_t e, const char* what, const char* file, int lin
 
 // Ensure buffer `id` holds at least `bytes`; contents are not preserved.
 int ensure(Ctx* c, BufId id, size_t bytes);
+// The same for a buffer that the caller can do without: false, and no error
+// recorded, when there is no room.
+bool ensure_optional(Ctx* c, BufId id, size_t bytes);
 template <typename T>
 inline T* bp(Ctx* c, BufId id) { return reinterpret_cast<T*>(c->buf[id].p); }
 

@@ -888,9 +888,10 @@ int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* m
   if (bytes(form) > c->smem_optin) return DCU_OK;
   const size_t smem = bytes(form) - kPStatic;
   auto al = [](size_t v) { return (v + 255) & ~(size_t)255; };
-  const size_t nslot = sh.cluster ? 0 : sizeof(PSlot) * kPSlotSets * kPMaxBlocks;
+  const size_t nslot = form != P_GRID ? 0 : sizeof(PSlot) * kPSlotSets * kPMaxBlocks;
   const size_t vec = al(sizeof(double) * (size_t)plan.n);
-  DCU_TRY(ensure(c, B_PERSIST, al(sizeof(SolveOut)) + nslot + (sh.cluster ? 0 : 4 * vec)));
+  // (without room for its vectors the solve goes to the launches)
+  if (!ensure_optional(c, B_PERSIST, al(sizeof(SolveOut)) + nslot + (form == P_GRID ? 4 * vec : 0))) return DCU_OK;
   char* base = bp<char>(c, B_PERSIST);
   a.n = plan.n;
   a.nslices = plan.nslices;

@@ -47,6 +47,13 @@ int ensure(Ctx* c, BufId id, size_t bytes) {
   return DCU_OK;
 }
 
+bool ensure_optional(Ctx* c, BufId id, size_t bytes) {
+  const std::string err = c->err;
+  if (ensure(c, id, bytes) == DCU_OK) return true;
+  c->err = err;
+  return false;
+}
+
 // ---------------------------------------------------------------------------
 // Exclusive scan.  Each block scans 1024 elements (256 threads x 4), writes
 // its total; totals are scanned recursively and added back.  Deterministic.

@@ -2187,9 +2187,9 @@ int run_rows(Ctx* c, const SmallArgs& sa) {
   ga.in = sa.list;
   ga.in_count = ST_FB_COUNT;
   ga.limit = sa.max_ni >= SG_MMAX ? INT_MAX : sa.max_ni;
-  if (sa.max_ni > GroupA::RMAX) {
-    const size_t n = (size_t)std::max(1, sa.col_end - sa.col_start);
-    DCU_TRY(ensure(c, B_MIDLIST, sizeof(int) * 2 * n));
+  // (without room for the lists the larger sizes are left out)
+  const size_t n = (size_t)std::max(1, sa.col_end - sa.col_start);
+  if (sa.max_ni > GroupA::RMAX && ensure_optional(c, B_MIDLIST, sizeof(int) * 2 * n)) {
     ga.mid_list = bp<int>(c, B_MIDLIST);
     ga.wide_list = ga.mid_list + n;
   }
@@ -2214,6 +2214,12 @@ int run_rows_rest(Ctx* c, const SmallArgs& sa, int mid) {
   return launch_rows<T, GroupC>(c, ga);
 }
 
+// Scratch of hub_panels (B_HUBT): T of two panels, block counts of every panel.
+size_t hub_panel_bytes(int nh, int steps) {
+  const size_t np = (steps + HUB_PANEL - 1) / HUB_PANEL;
+  return 2 * sizeof(double) * HUB_PANEL * HUB_PANEL * nh + sizeof(int) * np * (nh + 1);
+}
+
 // The panels of all hubs (sorted by |J| descending): factor, then apply, per panel.
 int hub_panels(Ctx* c, const HubArgs& h, const std::vector<HubMeta>& hm, int steps) {
   const int nh = (int)hm.size(), np = (steps + HUB_PANEL - 1) / HUB_PANEL;
@@ -2232,7 +2238,6 @@ int hub_panels(Ctx* c, const HubArgs& h, const std::vector<HubMeta>& hm, int ste
   }
   const size_t tcount = (size_t)HUB_PANEL * HUB_PANEL * nh;
   const size_t tbytes = 2 * sizeof(double) * tcount;  // T of this panel and of the next one
-  DCU_TRY(ensure(c, B_HUBT, tbytes + sizeof(int) * pre.size()));
   double* tq = bp<double>(c, B_HUBT);
   int* dpre = reinterpret_cast<int*>(bp<char>(c, B_HUBT) + tbytes);
   DCU_CUDA(c, cudaMemcpyAsync(dpre, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice, c->stream));
@@ -2333,7 +2338,7 @@ int run_large(Ctx* c, LargeArgs& a, int nbig, int cta_max_area = 0) {
   if constexpr (std::is_same<T, double>::value) {
     int tall = 1;
     for (const HubMeta& g : hm) tall = std::max(tall, g.m);
-    if (tall <= HUB_TALL) {
+    if (tall <= HUB_TALL && ensure_optional(c, B_HUBT, hub_panel_bytes(nh, steps))) {
       DCU_TRY(hub_panels(c, h, hm, steps));
       k_hub_solve<T><<<nh, LG_BLOCK, 0, c->stream>>>(h, a);
       DCU_LAUNCHED(c, "k_hub_solve");
