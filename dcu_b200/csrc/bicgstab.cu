@@ -591,8 +591,8 @@ __global__ void __launch_bounds__(BI_BLOCK, 8) k_bi_y(BiArgs<MT, IT, VT> a) {
 
 // K2: ay = A y; alpha = rho / (r*, ay)
 // 32 registers (8 blocks per SM) with 16-bit columns and a narrow M; with
-// int32 columns or an FP64 M up to 48 (5 blocks; K4 alike, 56 without the
-// bound).  At 8 blocks the FP64 form gains 0.4% at 128^3 and loses 9% at 75^3.
+// int32 columns or an FP64 M up to 48 (5 blocks).  At 8 blocks the FP64 form
+// gains 0.4% at 128^3 and loses 9% at 75^3.
 // (An explicit minimum of one block lets the compiler take 64 for the former.)
 template <typename MT, typename IT, typename VT>
 __global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || std::is_same<IT, int>::value) ? 5 : 8)
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || 
     v[0] += rsv * ayv;
   };
   const VT* __restrict__ rs = a.rs;
-  if (a.S->a32) {
+  if (a.aval32 && a.S->a32) {
     for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
       const double rsv = ldv(rs + r);
       row(r, rsv, a_row32(a, r, yf));
@@ -651,9 +651,21 @@ __global__ void __launch_bounds__(BI_BLOCK) k_bi_sz(BiArgs<MT, IT, VT> a) {
 }
 
 // K4: az = A z; omega = (az, s) / (az, az)
+// BLOCKS: resident blocks an SM the compiler is held to (0: not held).  8 with
+// 16-bit columns and a narrow M (32 registers).  Else, with FP64 vectors, 56
+// registers (4 blocks) when not held, 48 with some spills at 5 blocks, which
+// pays where the iteration is bound by HBM: 4 / 5 blocks, us an iteration, 190^3
+// FP64 506 / 496, BF16 M 430 / 421, 128^3 FP64 162.7 / 160.9; 75^3 FP64 61.6 /
+// 65.1, 700^2 55.4 / 57.2.  With FP32 vectors 48 either way, 8 bytes spilled
+// against 88 (circuit-like matrix of 60000 rows 190 / 197).
 template <typename MT, typename IT, typename VT>
-__global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || std::is_same<IT, int>::value) ? 5 : 8)
-    k_bi_az(BiArgs<MT, IT, VT> a) {
+constexpr int az_blocks(bool many) {
+  if (!std::is_same<MT, double>::value && !std::is_same<IT, int>::value) return 8;
+  return many && std::is_same<VT, double>::value ? 5 : 0;
+}
+constexpr long long kFiveBlocksNnz = 1ll << 22;
+template <typename MT, typename IT, typename VT, int BLOCKS>
+__global__ void __launch_bounds__(BI_BLOCK, BLOCKS) k_bi_az(BiArgs<MT, IT, VT> a) {
   if (finished(a.S)) return;
   double v[2] = {0.0, 0.0};
   const VT* __restrict__ z = a.z;
@@ -667,7 +679,7 @@ __global__ void __launch_bounds__(BI_BLOCK, (std::is_same<MT, double>::value || 
     v[1] += azv * azv;
   };
   const double* __restrict__ s = a.s;
-  if (a.S->a32) {
+  if (a.aval32 && a.S->a32) {
     for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
       const double sv = ldv(s + r);
       row(r, sv, a_row32(a, r, zf));
@@ -766,7 +778,7 @@ __global__ void __launch_bounds__(BI_BLOCK, 6) k_bi_xr(BiArgs<MT, IT, VT> a) {
 template <typename MT, typename IT, typename VT>
 __global__ void __launch_bounds__(BI_BLOCK) k_bi_true(BiArgs<MT, IT, VT> a, int replace) {
   double v[2] = {0.0, 0.0};
-  const bool a32 = a.S->a32;  // (k_bi_init decided it)
+  const bool a32 = a.aval32 && a.S->a32;  // (k_bi_init decided it)
   auto xf = [&](int c) { return ldv(a.x + c); };
   const int stride = gridDim.x * BI_BLOCK;
   for (int r = blockIdx.x * BI_BLOCK + threadIdx.x; r < a.n; r += stride) {
@@ -838,13 +850,15 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
     }
     return per_sm;
   };
+  const auto k_az = (long long)plan.nnz >= kFiveBlocksNnz ? k_bi_az<MT, IT, VT, az_blocks<MT, IT, VT>(true)>
+                                                          : k_bi_az<MT, IT, VT, az_blocks<MT, IT, VT>(false)>;
   std::array<int, IK_COUNT> rs;
   rs[IK_P] = resident((const void*)k_bi_p<MT, IT, VT>);
   rs[IK_Y] = resident((const void*)k_bi_y<MT, IT, VT>);
   rs[IK_PY] = resident((const void*)k_bi_py<MT, IT, VT>);
   rs[IK_AY] = resident((const void*)k_bi_ay<MT, IT, VT>);
   rs[IK_SZ] = resident((const void*)k_bi_sz<MT, IT, VT>);
-  rs[IK_AZ] = resident((const void*)k_bi_az<MT, IT, VT>);
+  rs[IK_AZ] = resident((const void*)k_az);
   rs[IK_XR] = resident((const void*)k_bi_xr<MT, IT, VT>);
   // rows each kernel's threads stride over (the p pass takes row pairs); the
   // kernels that end in a reduction keep one full wave over n, whatever the
@@ -932,7 +946,7 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
   }
   c->profile_k1_free = k1_free;
   c->profile_default_split = dsplit ? 1 : 0;
-  c->profile_launch = [c, a, grid_of](int kind, int s) -> int {
+  c->profile_launch = [c, a, grid_of, k_az](int kind, int s) -> int {
     const int g = grid_of(kind, s);
     DCU_CUDA(c, cudaMemsetAsync(&a.S->done, 0, sizeof(int), c->stream));
     switch (kind) {
@@ -941,7 +955,7 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
       case IK_PY: k_bi_py<MT, IT, VT><<<g, BI_BLOCK, 0, c->stream>>>(a); break;
       case IK_AY: k_bi_ay<MT, IT, VT><<<g, BI_BLOCK, 0, c->stream>>>(a); break;
       case IK_SZ: k_bi_sz<MT, IT, VT><<<g, BI_BLOCK, 0, c->stream>>>(a); break;
-      case IK_AZ: k_bi_az<MT, IT, VT><<<g, BI_BLOCK, 0, c->stream>>>(a); break;
+      case IK_AZ: k_az<<<g, BI_BLOCK, 0, c->stream>>>(a); break;
       default: k_bi_xr<MT, IT, VT><<<g, BI_BLOCK, 0, c->stream>>>(a); break;
     }
     DCU_LAUNCHED(c, "profile kernel");
@@ -990,7 +1004,7 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
   const int chunk = (long long)plan.nnz >= kChunkShortNnz ? kChunkShort : kChunkLong;
   // the key names the kernel instantiation too: the same buffers are reused
   // by every precision form
-  std::vector<const void*> key = {(const void*)&k_bi_py<MT, IT, VT>, (const void*)(intptr_t)grid,
+  std::vector<const void*> key = {(const void*)&k_bi_py<MT, IT, VT>, (const void*)k_az, (const void*)(intptr_t)grid,
                                   (const void*)(intptr_t)split,
                                   (const void*)(intptr_t)g_py, (const void*)(intptr_t)g_ay, (const void*)(intptr_t)g_sz,
                                   (const void*)(intptr_t)g_az, (const void*)(intptr_t)g_xr, (const void*)(intptr_t)g_p,
@@ -1021,7 +1035,7 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
       pre(k_bi_wide<MT, IT, VT, WIDE_SZ>);
       if (le == cudaSuccess) le = launch_pdl(k_bi_sz<MT, IT, VT>, g_sz, c->stream, a);
       pre(k_bi_wide<MT, IT, VT, WIDE_AZ>);
-      if (le == cudaSuccess) le = launch_pdl(k_bi_az<MT, IT, VT>, g_az, c->stream, a);
+      if (le == cudaSuccess) le = launch_pdl(k_az, g_az, c->stream, a);
       if (le == cudaSuccess) le = launch_pdl(k_bi_xr<MT, IT, VT>, g_xr, c->stream, a);
     }
     cudaError_t e = cudaStreamEndCapture(c->stream, &g);
