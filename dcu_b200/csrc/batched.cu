@@ -593,8 +593,6 @@ struct BCArgs {
   int* head;                // [0] taken, [1] from the front, [2] from the back
   const int* sys_off;
   const long long* off;
-  const int* kd;
-  const int* su;
   const int* ix;
   const double* aval;
   const double* mval;
@@ -671,7 +669,6 @@ template <int R>
 struct BCRows {
   static constexpr int V = vals_per_thread<R>(), T = R / V, ROWS = BCEntries<R>::ROWS;
   BCEntries<R>& E;
-  const long long* off;
   const int* ix;
   int c0, rows, sl0;
   long long ob;   // first slot of the CTA's first slice
@@ -828,7 +825,7 @@ __global__ void __launch_bounds__(BC_THREADS, 1) k_batch_cluster(BCArgs a) {
     __syncthreads();
     const int npass = (rpc + ROWS - 1) / ROWS;
     const int jr = tid / T;        // this thread's row of a pass
-    const BCRows<R> rw{E, a.off, a.ix, c0, rows, sl0, ob};
+    const BCRows<R> rw{E, a.ix, c0, rows, sl0, ob};
     rw.begin(a.aval);
 
     // r = b - A x, r* = r, q = 0
@@ -1221,8 +1218,6 @@ int run_batch_clusters(Ctx* c, int nsys, const int* sys_off_d, const std::vector
   BCArgs a{};
   a.sys_off = sys_off_d;
   a.off = plan.off;
-  a.kd = plan.kd;
-  a.su = plan.su;
   a.ix = plan.idx;
   a.aval = aval;
   a.mval = mval;
