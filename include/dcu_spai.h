@@ -315,8 +315,10 @@ int dcu_sell_plan_stats(dcu_spai_ctx* ctx, long long* slots, long long* uniform_
 int dcu_set_wide_prepass(dcu_spai_ctx* ctx, int enabled);
 
 /* Let this context's later solves in the forms other than DCU_PREC_FP64, and
- * in DCU_PREC_FP64 from 2^22 stored slots on, read A's values from an FP32 copy when every value of A is exactly an FP32
- * number (enabled != 0, the default), or always from the FP64 array (0).
+ * in DCU_PREC_FP64 from 2^22 stored slots on, read A's values from an FP32
+ * copy when every value of A is exactly an FP32 number (enabled != 0, the
+ * default), or always from the FP64 array (0; also plain FP64 where there is no
+ * room for the copy, and batched solves).
  * The check runs on the device while A is laid out for the solver; the
  * products are formed in FP64 from the same numbers either way, so the
  * iterates are bit-identical, and a matrix with one value that FP32 rounds
@@ -334,17 +336,18 @@ int dcu_set_exact_a32(dcu_spai_ctx* ctx, int enabled);
  * on the grid, and the two first steps compute the same values, so every
  * field except group_max_ni leaves the solution bit-identical:
  *   k1_split   -1: the form's default (split with an FP32 / BF16 M and, from
- *              2^22 entries on, with an FP64 M; else fused); 0: fused (p formed at every gathered column
- *              inside y = M p); 1: split (a p pass, then y = M p).  Forms with
+ *              2^22 entries on, with an FP64 M; else fused); 0: fused (p formed
+ *              at every gathered column inside y = M p); 1: split (a p pass, then y = M p).  Forms with
  *              FP32 vectors keep their default: their fused step multiplies
  *              by the unrounded p, so the two differ in rounding there.
  *   grid_p, grid_y, grid_py, grid_sz   the kernels without a reduction:
  *              p pass, y = M p, fused p/y, s/z = M s.  The kernels that end
  *              in a dot product keep one full wave: their grid fixes the
  *              summation order of the partial sums.
- *   group_max_ni   SPAI build: largest |I_k| the warp-group (warp-per-small)
- *              kernel takes, 1..32 (0 = 32); larger columns go to the
- *              CTA-per-column kernel.  Changes M by rounding only.
+ *   group_max_ni   SPAI build: largest |I_k| the lane-group kernels take, 1..31;
+ *              larger columns, and with a limit those of |J_k| > 7 or over 64
+ *              candidates, go to the CTA-per-column kernel.  0 or 32: no limit
+ *              but the kernels' own.  Changes M by rounding only.
  *   cta_max_area   SPAI build: largest dense block |I_k| x (|J_k| + 1) one CTA
  *              factors; a larger block is gathered into its own slab and
  *              factored by the hub kernels, every SM on every such column.
