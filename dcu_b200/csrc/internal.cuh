@@ -216,6 +216,7 @@ struct SellPlan {
   // when there is no such shape
   int max_block_slots[2] = {0, 0}, max_block_long[2] = {0, 0};
   long long uniform_slots = 0;  // slots in offset-uniform slices
+  int remote = 0;  // with two shapes: slots whose column lies in another block of the first
 };
 
 // How the one-launch solver splits an operator of n rows: `blocks` blocks

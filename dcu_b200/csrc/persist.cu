@@ -827,7 +827,10 @@ PersistShape persist_shape(const Ctx* c, int n, bool second) {
   const int nslices = (n + 31) / 32;
   int k = 1;
   const bool one_cluster = nslices <= 16 * 32;
-  if (second && !one_cluster) return s;
+  // (below 13 blocks of 512 rows the grid form is no faster than the cluster's 16
+  // CTAs: circuit-like matrix of 5600 rows, FP64, 5.08 against 4.96 ms; random
+  // columns, 7000 rows, 0.62 against 0.70)
+  if (second && (!one_cluster || nslices <= 192)) return s;
   // cluster form: up to 16 CTAs of up to 1024 rows; fewer CTAs while 256 rows each
   if (one_cluster && !second) {
     while (k < 16 && (nslices + k - 1) / k > 8) k <<= 1;
@@ -866,22 +869,28 @@ int persist_solve(Ctx* c, const SellPlan& plan, const SellA& aval, const void* m
   // Scattered columns (fewer than half the slots in slices of one offset a
   // position): a gather of 32 scattered elements through distributed shared
   // memory goes lane by lane, so each row is written to every CTA instead and
-  // gathered locally, where the whole vectors fit; else through L2 in the grid
-  // form.  Random columns, 5 a row, BF16 M, whole calls, launches / pull / grid:
-  // 10000 rows 1.18 / 0.95 / 0.72 ms, 14000 0.95 / 1.12 / 0.70.
+  // gathered locally, where the whole vectors fit.  Else, where a third of the
+  // entries lie in another CTA's rows (or the cluster does not hold the
+  // operator), through L2 in the grid form.  Random columns, 5 a row, BF16 M, whole
+  // calls, launches / pull / grid: 10000 rows 1.18 / 0.95 / 0.72 ms, 14000 0.95 /
+  // 1.12 / 0.70; columns within 300 rows (12000 rows, a fifth remote) pull / grid
+  // 0.51 / 0.56, within 1200 (two thirds) 0.79 / 0.67.
   int form = sh.cluster ? P_PULL : P_GRID;
   if (sh.cluster && 2 * plan.uniform_slots < plan.slots) {
     if (rows <= 512 && bytes(P_PUSH) <= c->smem_optin) {
       form = P_PUSH;
     } else {
       const PersistShape first = sh;
-      sh = persist_shape(c, plan.n, true);
-      take(1);
-      form = P_GRID;
-      if (bytes(form) > c->smem_optin) {
-        sh = first;
-        take(0);
-        form = P_PULL;
+      const bool holds = bytes(P_PULL) <= c->smem_optin;
+      if (!holds || 3ll * plan.remote >= plan.nnz) {
+        sh = persist_shape(c, plan.n, true);
+        take(1);
+        form = P_GRID;
+        if (bytes(form) > c->smem_optin) {
+          sh = first;
+          take(0);
+          form = P_PULL;
+        }
       }
     }
   }

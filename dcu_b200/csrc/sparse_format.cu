@@ -341,13 +341,15 @@ __global__ void k_sell_width(const int* __restrict__ rptr, int n, int nslices, i
 //     (wide) for a full slice wider than kWideSlice made so by at most
 //     kWideRows long rows, listed in wide (wide[0] counts);
 //   *uslots += the slots of the uniform slices (one atomic per block).
-__global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restrict__ rcol,
+// SECOND: the one-launch solver has a second shape for the operator.
+template <bool SECOND>
+__global__ void __launch_bounds__(256, SECOND ? 4 : 5) k_sell_layout(const int* __restrict__ rptr, const int* __restrict__ rcol,
                               const int* __restrict__ rperm, int n, int nslices, const long long* __restrict__ off,
                               int* __restrict__ sidx, int* __restrict__ sperm, int* __restrict__ maxdelta,
                               int16_t* __restrict__ del, int* __restrict__ kd, int* __restrict__ su,
                               unsigned long long* __restrict__ uslots, int* __restrict__ wide, int allow_wide,
                               int* __restrict__ kd8, int16_t* __restrict__ kd8h, int* __restrict__ cost, int spb,
-                              int* __restrict__ cost2, int spb2) {
+                              int* __restrict__ cost2, int spb2, int* __restrict__ remote) {
   __shared__ unsigned long long blk_uslots;
   if (threadIdx.x == 0) blk_uslots = 0ull;
   __syncthreads();
@@ -368,9 +370,14 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
     for (int j = 0; j < len; ++j) local_max = max(local_max, abs(rcol[rs + j] - self));
     bool all = true;
     int my_d = 0;  // lane k < kNarrow: offset of entry position k
+    // this row's slots whose column lies outside the rows of its block (first shape)
+    const int blk0 = SECOND ? s / spb * spb * 32 : 0;
+    const unsigned blkn = SECOND ? (unsigned)spb * 32u : 0u;
+    int far = 0;
     // slot k of this row holds column col: its delta and the slice's offset check
     auto note = [&](int k, long long q, int col) {
       del[q] = (int16_t)(col - self);
+      if (SECOND) far += (unsigned)(col - blk0) >= blkn;
       const int d = col - r;
       const int d0 = __shfl_sync(0xffffffffu, d, 0);  // row 32 s < n always
       const bool same = __all_sync(0xffffffffu, r >= n || d == d0);
@@ -405,6 +412,7 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
     if (sparse || !__all_sync(0xffffffffu, i == len)) {
       all = true;
       my_d = 0;
+      far = 0;
       for (int k = 0; k < w; ++k) {
         const long long q = base + 32ll * k;
         int col;
@@ -433,10 +441,12 @@ __global__ void k_sell_layout(const int* __restrict__ rptr, const int* __restric
       const int ws = __reduce_max_sync(0xffffffffu, !split ? w : (len <= kPersistLong ? len : 0));
       const int le = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? len : 0);
       const int nl = __reduce_add_sync(0xffffffffu, split && len > kPersistLong ? (len + kPersistSeg - 1) / kPersistSeg : 0);
+      const int nfar = SECOND ? __reduce_add_sync(0xffffffffu, r < n ? far : 0) : 0;
       if (lane == 0) {
         atomicAdd(&cost[2 * (s / spb)], 32 * ws + le);
         if (nl) atomicAdd(&cost[2 * (s / spb) + 1], nl);
-        if (spb2 > 0) {
+        if (SECOND) {
+          if (nfar) atomicAdd(remote, nfar);
           atomicAdd(&cost2[2 * (s / spb2)], 32 * ws + le);
           if (nl) atomicAdd(&cost2[2 * (s / spb2) + 1], nl);
         }
@@ -774,8 +784,8 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   // segments of long rows
   const PersistShape ps[2] = {persist_shape(c, n), persist_shape(c, n, true)};
   const int nblocks = ps[0].blocks + ps[1].blocks;  // (16 + 32 at most where there is a second shape)
-  unsigned long long hst[2 + kPersistBlocks] = {(unsigned long long)slots};
-  const size_t nst = sizeof(unsigned long long) * (2 + (size_t)nblocks);
+  unsigned long long hst[3 + kPersistBlocks] = {(unsigned long long)slots};
+  const size_t nst = sizeof(unsigned long long) * (3 + (size_t)nblocks);  // (the last one: remote slots)
   DCU_TRY(ensure(c, B_PLANSTAT, sizeof(hst)));
   unsigned long long* pst = bp<unsigned long long>(c, B_PLANSTAT);
   int* cost = reinterpret_cast<int*>(pst + 2);
@@ -786,14 +796,15 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
   int* kd8 = bp<int>(c, B_SELL_KD8);
   int16_t* kd8h = reinterpret_cast<int16_t*>(kd8 + kNarrow * (size_t)nslices);
   DCU_CUDA(c, cudaMemsetAsync(wide, 0, sizeof(int), c->stream));
-  k_sell_layout<<<waves_grid(c, (long long)nslices * 32, 256, 8), 256, 0, c->stream>>>(
+  const auto layout = ps[1].blocks > 0 ? k_sell_layout<true> : k_sell_layout<false>;
+  layout<<<waves_grid(c, (long long)nslices * 32, 256, 8), 256, 0, c->stream>>>(
       rptr, rcol, rperm, n, nslices, off, sidx, sperm, maxdelta, del, kd, su, pst + 1, wide, c->wide_prepass ? 1 : 0,
-      kd8, kd8h, cost, ps[0].blocks > 0 ? ps[0].spb : 0, cost + 2 * ps[0].blocks, ps[1].blocks > 0 ? ps[1].spb : 0);
+      kd8, kd8h, cost, ps[0].blocks > 0 ? ps[0].spb : 0, cost + 2 * ps[0].blocks, ps[1].spb, cost + 2 * nblocks);
   DCU_LAUNCHED(c, "k_sell_layout");
   // [0] wide slices, [1] largest delta, [2] check, then uniform slots and the blocks' costs
   int* hcost = reinterpret_cast<int*>(c->pinned) + 4;
-  static_assert(sizeof(int) * (6 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
-  DCU_CUDA(c, cudaMemcpyAsync(hcost, pst + 1, sizeof(unsigned long long) * (1 + (size_t)nblocks),
+  static_assert(sizeof(int) * (8 + 2 * kPersistBlocks) <= kPinnedBytes, "pinned scratch");
+  DCU_CUDA(c, cudaMemcpyAsync(hcost, pst + 1, sizeof(unsigned long long) * (2 + (size_t)nblocks),
                               cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(c->pinned, wide, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   DCU_CUDA(c, cudaMemcpyAsync(reinterpret_cast<int*>(c->pinned) + 1, maxdelta, sizeof(int), cudaMemcpyDeviceToHost,
@@ -813,6 +824,7 @@ int sell_fill_from_csr(Ctx* c, int n, int nnz, const int* rptr, const int* rcol,
       plan->max_block_long[k] = std::max(plan->max_block_long[k], hcost[1]);
     }
   }
+  plan->remote = *hcost;
   plan->delta16 = reinterpret_cast<int*>(c->pinned)[1] < 32768;
   plan->del = plan->delta16 ? del : nullptr;
   if (!plan->delta16) kd8h = nullptr;
