@@ -984,8 +984,9 @@ int run_solver(Ctx* c, const SellPlan& plan, const SellA& aval, const MT* mval, 
       // the profiling launches start from clean scalars and counters, and read A
       // as the solve did: its FP64 array may be absent (not waited for)
       DCU_CUDA(c, cudaMemsetAsync(a.S, 0, sizeof(Scal), c->stream));
-      DCU_CUDA(c, cudaMemcpyAsync(&a.S->a32, &bp<SolveOut>(c, B_PERSIST)->a32, sizeof(int), cudaMemcpyDeviceToDevice,
-                                  c->stream));
+      if (o.a32)
+        DCU_CUDA(c, cudaMemcpyAsync(&a.S->a32, &bp<SolveOut>(c, B_PERSIST)->a32, sizeof(int), cudaMemcpyDeviceToDevice,
+                                    c->stream));
       return DCU_OK;
     }
   }
