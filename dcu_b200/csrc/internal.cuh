@@ -221,7 +221,8 @@ struct SellPlan {
 
 // How the one-launch solver splits an operator of n rows: `blocks` blocks
 // (0: too large for it) of `spb` 32-row slices each.  An operator for one
-// cluster has a second shape, the grid form (for scattered columns).
+// cluster has a second shape from 6145 rows on, the grid form (for scattered
+// columns).
 struct PersistShape {
   bool cluster = false;
   int spb = 0, blocks = 0;
